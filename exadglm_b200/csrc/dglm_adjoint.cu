@@ -1178,7 +1178,7 @@ cudaError_t frozen_stage(dglm_handle *h, const double *u_in, double *u_out, doub
   a.tau = tau;
   a.dt_override = dt;
   a.last_stage = 0;
-  return launch_stage_fp64(h->d.physics, h->d.N, h->variant, a, cs);
+  return launch_stage_fp64(h->d.physics, h->d.N, h->run_variant, a, cs);
 }
 
 // ---- binomial checkpointing under a memory cap ------------------------------

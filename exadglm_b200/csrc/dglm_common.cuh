@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <vector>
 
 #include "dglm.h"
 
@@ -176,7 +177,8 @@ dglm_status cuda_check(cudaError_t e, const char *what);
 
 // contraction engines of the fused stage kernel
 enum { MODE_SIMT = 0, MODE_DMMA = 1, MODE_PIPE = 2, MODE_MIXED = 3, MODE_MMA16 = 4, MODE_TC = 5,
-       MODE_TCB = 6 };
+       MODE_TCB = 6,
+       MODE_SYM = 7 };
 
 // One compiled tile shape of the fused stage kernel.
 struct StageVariantInfo {
@@ -204,7 +206,30 @@ struct StageVariantInfo {
   int k_global;    // PIPE: 1 = the RK register is fetched by the update, not staged
   int op_global;   // PIPE: 1 = operator fragments read through L1, not staged in shared memory
   int ctas_per_sm; // PIPE: persistent CTAs per SM (2: two independent pipelines per SM)
+  int fallback;    // SYM: variant that runs when the operators lack the symmetry
 };
+
+// One entry of the variant tables: a tile shape and its launcher.
+struct StageVariant {
+  StageVariantInfo info;
+  cudaError_t (*launch)(const StageArgs &, cudaStream_t);
+};
+
+// Symmetry-adapted Euler stage (dglm_stage_sym.cu), orders 3..6.
+StageVariant sym_variant(int N, int fallback);
+// Its operator image from A = [WDr WDs WDt -LIFT] (Np rows, row-major); false
+// when the operators or Fmask lack the symmetry of the reference tetrahedron.
+bool sym_operator_image(int N, const double *A, const int *Fmask, std::vector<double> &img);
+// Element records (kRecord) of Kp elements from the uploaded metrics [9][Kp],
+// normals [3][4Kp] and Fscale, on the legacy stream; sym: as the
+// symmetry-adapted kernel takes them (metrics in the gauge that leaves out
+// vertex 0, grad r_a + sum_b grad r_b; normals times Fscale / 2, and Fscale / 2).
+cudaError_t launch_element_records(const double *geo, const double *nrm, const double *fscale,
+                                   long Kp, bool sym, double *rec);
+// RK register of `tiles` tiles of 8 elements: nodal order (variable blocks of
+// vs doubles) to the kernel's fragment order, or back (out zeroed by the caller).
+void sym_reorder_register(int N, long tiles, int nvar, long vs, const double *in, double *out,
+                          bool to_sym);
 
 // fused FP64 stage launcher (dglm_stage_fp64.cu)
 bool stage_fp64_supported(int physics, int N);

@@ -14,9 +14,13 @@ struct AdjointTape;
 struct dglm_handle {
   dglm_desc d{};
   int nvar = 0, Np = 0, Nfp = 0, NFF = 0;
-  int variant = 0;
-  dglm::StageVariantInfo vinfo{};
+  int variant = 0;                // selected by the caller
+  int run_variant = 0;            // launched: the selected one, or its fallback when the
+                                  // uploaded operators lack the symmetry it needs
+  dglm::StageVariantInfo vinfo{}; // of run_variant
+  bool op_symmetric = true;       // whether the uploaded operators have that symmetry
   std::vector<double> Ahost;      // stacked [WDr WDs WDt -LIFT], Np x (3Np+NFF) row-major
+  std::vector<double> sym_image;  // operator image of the symmetry-adapted kernel
   long vs = 0;                    // doubles between variables of a field
   long Kp = 0;                    // K rounded up to a multiple of 64 (tile padding)
   int dev = 0;
@@ -26,9 +30,9 @@ struct dglm_handle {
   double *AT = nullptr, *geo = nullptr, *fscale = nullptr, *nrm = nullptr;
   double *tau = nullptr, *maxv = nullptr, *vel = nullptr;
   int *vmapP = nullptr, *vmapF = nullptr, *Fmask = nullptr;
-  // per-element record [Kp][kRecord] (TF32x3 and BF16x3 Euler handles): the 9 metrics,
+  // per-element record [Kp][kRecord] (Euler handles but BF16x6): the 9 metrics,
   // nx, ny, nz and Fscale of the 4 faces, one pad double; one bulk copy per
-  // tile in the tensor-memory kernel
+  // tile in the tensor-memory and symmetry-adapted kernels
   double *erec = nullptr;
   // compact face maps (dglm_set_compact_face_maps), built from vmapP on first
   // use: per face the neighbour element and a code of its node list

@@ -94,7 +94,7 @@ namespace {
 // Doubles of the device operator copy for a variant's layout.
 size_t op_doubles(const StageVariantInfo &v, int Np, int NFF) {
   if (v.mode == MODE_SIMT) return (size_t)(3 * Np + NFF) * v.IP;
-  if (v.mode == MODE_MIXED || v.mode == MODE_TC || v.mode == MODE_TCB)
+  if (v.mode == MODE_MIXED || v.mode == MODE_TC || v.mode == MODE_TCB || v.mode == MODE_SYM)
     return ((size_t)v.bimg + 7) / 8;
   if (v.mode == MODE_MMA16) {
     const int parts = v.prec == DGLM_PREC_BF16X6 ? 3 : 2;
@@ -308,6 +308,11 @@ dglm_status upload_operator_layout(dglm_handle *h) {
     return cuda_check(cudaMemcpy(h->AT, img.data(), img.size() * 4, cudaMemcpyHostToDevice),
                       "operator upload");
   }
+  if (v.mode == MODE_SYM) {
+    return cuda_check(cudaMemcpy(h->AT, h->sym_image.data(),
+                                 sizeof(double) * h->sym_image.size(), cudaMemcpyHostToDevice),
+                      "operator upload");
+  }
   if (v.mode == MODE_MMA16) {
     std::vector<uint32_t> fr = m16_fragments(h, v);
     return cuda_check(cudaMemcpy(h->AT, fr.data(), fr.size() * 4, cudaMemcpyHostToDevice),
@@ -347,6 +352,32 @@ dglm_status upload_operator_layout(dglm_handle *h) {
                     "operator upload");
 }
 
+// The variant to launch for the selected one: a symmetry-adapted variant needs
+// operators with the symmetry of the reference tetrahedron (every symmetric
+// node set's have it); others run on its fallback.
+void choose_run_variant(dglm_handle *h) {
+  StageVariantInfo v{};
+  stage_variant_info(h->d.physics, h->d.N, h->variant, &v);
+  h->run_variant = v.mode == MODE_SYM && !h->op_symmetric ? v.fallback : h->variant;
+  stage_variant_info(h->d.physics, h->d.N, h->run_variant, &h->vinfo);
+}
+
+// Brings the RK register into the run variant's order after a change of
+// variant in the middle of a step (symmetry-adapted kernels keep it in
+// fragment order, the others in nodal order).  Host copies: a caller switches
+// variants between stages, if at all, once.
+dglm_status convert_register(dglm_handle *h, int from_mode) {
+  if ((from_mode == MODE_SYM) == (h->vinfo.mode == MODE_SYM)) return DGLM_OK;
+  const size_t n = (size_t)h->nvar * h->vs;
+  std::vector<double> in(n), out(n, 0.0);
+  cudaError_t e = cudaMemcpy(in.data(), h->kreg, sizeof(double) * n, cudaMemcpyDeviceToHost);
+  if (e != cudaSuccess) return cuda_check(e, "RK register");
+  sym_reorder_register(h->d.N, (h->d.K + 7) / 8, h->nvar, h->vs, in.data(), out.data(),
+                       h->vinfo.mode == MODE_SYM);
+  e = cudaMemcpy(h->kreg, out.data(), sizeof(double) * n, cudaMemcpyHostToDevice);
+  return cuda_check(e, "RK register");
+}
+
 // Whether the step's wave-speed maximum runs as its own kernel after the
 // fifth stage (Euler): inside the persistent stage kernels it costs more than
 // the standalone face_maxv_kernel, whose result is the same bit for bit.
@@ -373,7 +404,7 @@ dglm_status dglm::issue_step_ptrs(dglm_handle *h, const double *const *in, doubl
   for (int st = 0; st < 5 && e == cudaSuccess; st++) {
     StageArgs a = stage_args(h, in[st], out[st], st);
     if (sep) a.last_stage = 0;
-    e = launch_stage_fp64(h->d.physics, h->d.N, h->variant, a, s);
+    e = launch_stage_fp64(h->d.physics, h->d.N, h->run_variant, a, s);
   }
   if (e == cudaSuccess && sep)
     e = launch_face_maxv(h->d.physics, h->d.N, stage_args(h, out[4], nullptr, -1), -1, s);
@@ -394,7 +425,7 @@ dglm_status issue_step(dglm_handle *h, int cur, cudaStream_t s) {
     const int in = (cur + st) & 1;
     StageArgs a = stage_args(h, h->u[in], h->u[in ^ 1], st);
     if (sep) a.last_stage = 0;
-    e = launch_stage_fp64(h->d.physics, h->d.N, h->variant, a, s);
+    e = launch_stage_fp64(h->d.physics, h->d.N, h->run_variant, a, s);
   }
   // after five stages the new state is in u[cur ^ 1]
   if (e == cudaSuccess && sep)
@@ -481,7 +512,7 @@ dglm_status dglm_create(const dglm_desc *desc, dglm_handle **out) {
   h->Nfp = nfp_of(d.N);
   h->NFF = 4 * h->Nfp;
   h->variant = first;
-  stage_variant_info(d.physics, d.N, first, &h->vinfo);
+  choose_run_variant(h);
   // per-element arrays are padded to whole 64-element tiles (zero-filled) so
   // that every tile copy of the pipelined kernel is in bounds and aligned
   h->Kp = ((long)d.K + 63) / 64 * 64;
@@ -496,8 +527,7 @@ dglm_status dglm_create(const dglm_desc *desc, dglm_handle **out) {
   chk(dalloc(h, &h->geo, (size_t)9 * K));
   chk(dalloc(h, &h->fscale, (size_t)4 * K));
   chk(dalloc(h, &h->nrm, (size_t)12 * K));
-  if (d.physics == DGLM_EULER &&
-      (d.precision == DGLM_PREC_TF32X3 || d.precision == DGLM_PREC_BF16X3))
+  if (d.physics == DGLM_EULER && d.precision != DGLM_PREC_BF16X6)
     chk(dalloc(h, &h->erec, (size_t)kRecord * K));
   chk(dalloc(h, &h->tau, (size_t)4 * K));
   chk(dalloc(h, &h->maxv, (size_t)4 * K));
@@ -630,25 +660,18 @@ dglm_status dglm_upload_mesh(dglm_handle *h, const dglm_mesh_arrays *m) {
   cudaStreamSynchronize(h->stream);
   free_tape(h);   // the adjoint's operators and face pairing belong to the old mesh
   const auto H2D = cudaMemcpyHostToDevice;
+  h->op_symmetric = h->d.physics == DGLM_EULER && h->d.precision == DGLM_PREC_FP64 &&
+                    sym_operator_image(h->d.N, h->Ahost.data(), m->Fmask, h->sym_image);
+  choose_run_variant(h);
+  drop_graphs(h);
   dglm_status os = upload_operator_layout(h);
   if (os != DGLM_OK) return os;
   cudaError_t e = cudaMemcpy(h->geo, geo.data(), sizeof(double) * geo.size(), H2D);
   if (e == cudaSuccess) e = cudaMemcpy(h->nrm, nrm.data(), sizeof(double) * nrm.size(), H2D);
   if (e == cudaSuccess) e = cudaMemcpy(h->fscale, m->Fscale, sizeof(double) * 4 * K, H2D);
-  if (e == cudaSuccess && h->erec) {
-    std::vector<double> rec((size_t)kRecord * Kp, 0.0);
-    for (long k = 0; k < K; k++) {
-      double *r = &rec[(size_t)k * kRecord];
-      for (int q = 0; q < 9; q++) r[q] = g9[q][k];
-      for (int f = 0; f < 4; f++) {
-        r[9 + f] = m->nx[4 * k + f];
-        r[13 + f] = m->ny[4 * k + f];
-        r[17 + f] = m->nz[4 * k + f];
-        r[21 + f] = m->Fscale[4 * k + f];
-      }
-    }
-    e = cudaMemcpy(h->erec, rec.data(), sizeof(double) * rec.size(), H2D);
-  }
+  if (e == cudaSuccess && h->erec)
+    e = launch_element_records(h->geo, h->nrm, h->fscale, Kp,
+                               h->d.precision == DGLM_PREC_FP64, h->erec);
   if (e == cudaSuccess) e = cudaMemcpy(h->vmapP, m->vmapP, sizeof(int) * K * NFF, H2D);
   if (e == cudaSuccess) e = cudaMemcpy(h->vmapF, m->vmapF, sizeof(int) * 4 * K, H2D);
   if (e == cudaSuccess) e = cudaMemcpy(h->Fmask, m->Fmask, sizeof(int) * NFF, H2D);
@@ -918,7 +941,13 @@ dglm_status dglm_stage(dglm_handle *h, int stage, double dt) {
   DeviceGuard g(h->dev);
   StageArgs a = stage_args(h, h->u[h->cur], h->u[h->cur ^ 1], stage);
   a.dt_override = dt;
-  cudaError_t e = launch_stage_fp64(h->d.physics, h->d.N, h->variant, a, h->stream);
+  // the symmetry-adapted kernel leaves the wave speeds to the separate kernel
+  const bool sep = a.last_stage && h->vinfo.mode == MODE_SYM;
+  if (sep) a.last_stage = 0;
+  cudaError_t e = launch_stage_fp64(h->d.physics, h->d.N, h->run_variant, a, h->stream);
+  if (e == cudaSuccess && sep)
+    e = launch_face_maxv(h->d.physics, h->d.N, stage_args(h, a.u_out, nullptr, -1), -1,
+                         h->stream);
   if (e != cudaSuccess) return cuda_check(e, "dglm_stage");
   h->cur ^= 1;
   return DGLM_OK;
@@ -999,7 +1028,7 @@ dglm_status dglm_rhs(dglm_handle *h, const double *const *u, double *const *rhs)
   a.rhs_only = 1;
   if (e == cudaSuccess) e = launch_face_maxv(h->d.physics, h->d.N, a, 0, s);
   if (e == cudaSuccess) e = launch_tau(h->d.K, h->d.tau_scale, h->vmapF, h->maxv_s, h->tau_s, s);
-  if (e == cudaSuccess) e = launch_stage_fp64(h->d.physics, h->d.N, h->variant, a, s);
+  if (e == cudaSuccess) e = launch_stage_fp64(h->d.physics, h->d.N, h->run_variant, a, s);
   for (int v = 0; v < h->nvar && e == cudaSuccess; v++)
     e = cudaMemcpyAsync(rhs[v], h->rhs_out + (size_t)v * h->vs, sizeof(double) * n,
                         cudaMemcpyDeviceToDevice, s);
@@ -1019,7 +1048,10 @@ dglm_status dglm_variant_describe(int physics, int N, int variant, char *buf, si
   StageVariantInfo v{};
   if (!buf || len == 0 || !stage_variant_info(physics, N, variant, &v))
     return set_error(DGLM_ERR_INVALID, "dglm_variant_describe: no such variant");
-  if (v.mode == MODE_SIMT)
+  if (v.mode == MODE_SYM)
+    snprintf(buf, len, "pipe-dmma-sym E=%d groups=%d warps/group=%d threads=%d smem=%zu ring=%d", v.E,
+             v.groups, v.R, v.threads, v.smem, v.ring);
+  else if (v.mode == MODE_SIMT)
     snprintf(buf, len, "simt E=%d R=%d CPT=%d threads=%d smem=%zu", v.E, v.R, v.CPT, v.threads,
              v.smem);
   else if (v.mode == MODE_MMA16)
@@ -1081,10 +1113,12 @@ dglm_status dglm_set_variant(dglm_handle *h, int variant) {
   DeviceGuard g(h->dev);
   cudaStreamSynchronize(h->stream);
   drop_graphs(h);
+  const int from_mode = h->vinfo.mode;
   h->variant = variant;
-  h->vinfo = v;
-  if (h->mesh_ready) return upload_operator_layout(h);
-  return DGLM_OK;
+  choose_run_variant(h);
+  if (!h->mesh_ready) return DGLM_OK;
+  dglm_status st = h->state_ready ? convert_register(h, from_mode) : DGLM_OK;
+  return st == DGLM_OK ? upload_operator_layout(h) : st;
 }
 
 int dglm_get_variant(dglm_handle *h) { return h ? h->variant : -1; }

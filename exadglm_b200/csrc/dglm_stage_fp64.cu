@@ -40,6 +40,7 @@
 #include <vector>
 
 #include "dglm_common.cuh"
+#include "dglm_ptx.cuh"
 
 namespace dglm {
 
@@ -173,13 +174,6 @@ __device__ __forceinline__ void contract_simt(const double *__restrict__ AT, int
 #pragma unroll
       for (int j = 0; j < C::CPT; j++) acc[r][j] = fma(av[r], bv[j], acc[r][j]);
   }
-}
-
-__device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
-  asm volatile(
-      "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-      : "+d"(d[0]), "+d"(d[1])
-      : "d"(a), "d"(b));
 }
 
 // A fragments are stored [kstep][mtile][lane] in the lane order of the
@@ -784,10 +778,7 @@ __global__ void tau_kernel(int K, double tau_scale, const int *__restrict__ vmap
 // variants and dispatch
 // ---------------------------------------------------------------------------
 
-struct Variant {
-  StageVariantInfo info;
-  cudaError_t (*launch)(const StageArgs &, cudaStream_t);
-};
+using Variant = StageVariant;
 
 template <int PHYS, int N, int MODE, int E, int R, int CPT, int WM, int PR = 0>
 static cudaError_t launch_v(const StageArgs &a, cudaStream_t s) {
@@ -1037,11 +1028,11 @@ static const std::vector<Variant> &variants();
 
 DGLM_VARIANTS(EUL, 1, V_SIMT(EUL, 1, 128, 4, 5), V_DMMA(EUL, 1, 64, 4, 1))
 DGLM_VARIANTS(EUL, 2, V_SIMT(EUL, 2, 64, 5, 5), V_DMMA(EUL, 2, 32, 4, 2))
-DGLM_VARIANTS(EUL, 3, V_DMMA(EUL, 3, 16, 2, 3), V_SIMT(EUL, 3, 32, 5, 5),
+DGLM_VARIANTS(EUL, 3, sym_variant(3, 4), V_DMMA(EUL, 3, 16, 2, 3), V_SIMT(EUL, 3, 32, 5, 5),
               V_PIPE(EUL, 3, 8, 1, 3, true), V_PIPE(EUL, 3, 16, 1, 3, true),
               V_PIPEF(EUL, 3, 8, 1, true, 3, 2), V_PIPEF(EUL, 3, 16, 2, true, 3, 2),
               V_TC(EUL, 3, 8, 14, 3))
-DGLM_VARIANTS(EUL, 4, V_PIPE(EUL, 4, 8, 1, 2, true), V_DMMA(EUL, 4, 8, 1, 5),
+DGLM_VARIANTS(EUL, 4, sym_variant(4, 26), V_PIPE(EUL, 4, 8, 1, 2, true), V_DMMA(EUL, 4, 8, 1, 5),
               V_SIMT(EUL, 4, 16, 5, 5), V_SIMT(EUL, 4, 16, 3, 5), V_DMMA(EUL, 4, 16, 1, 5),
               V_DMMA(EUL, 4, 16, 2, 5), V_PIPE(EUL, 4, 8, 1, 5, true),
               V_PIPE(EUL, 4, 8, 1, 5, false), V_PIPE(EUL, 4, 8, 1, 3, true),
@@ -1056,13 +1047,13 @@ DGLM_VARIANTS(EUL, 4, V_PIPE(EUL, 4, 8, 1, 2, true), V_DMMA(EUL, 4, 8, 1, 5),
               V_PIPE2C(EUL, 4, 8, 5, 1, 2, 1), V_PIPE2C(EUL, 4, 8, 1, 5, 2, 2),
               V_TC(EUL, 4, 8, 14, 3), V_TCB(EUL, 4, 8, 14, 2, true),
               V_TC2(EUL, 4, 8, 13, 3), V_TCD(EUL, 4, 8, 14, 3))
-DGLM_VARIANTS(EUL, 5, V_PIPE(EUL, 5, 8, 1, 7, false), V_DMMA(EUL, 5, 8, 1, 7),
+DGLM_VARIANTS(EUL, 5, sym_variant(5, 10), V_PIPE(EUL, 5, 8, 1, 7, false), V_DMMA(EUL, 5, 8, 1, 7),
               V_SIMT(EUL, 5, 8, 7, 5), V_M16(EUL, 5, 8, 1, 2, 2), V_M16(EUL, 5, 8, 1, 2, 1),
               V_M16(EUL, 5, 8, 1, 2, 3), V_PIPEF(EUL, 5, 8, 1, false, 3, 2),
               V_PM16G(EUL, 5, 8, 1, 2, 1, 2), V_PIPEFW(EUL, 5, 8, 5, 1, false, 1, 2),
               V_PIPEFW(EUL, 5, 8, 5, 1, false, 2, 2), V_PIPEFW(EUL, 5, 8, 5, 2, false, 3, 2),
               V_TCB(EUL, 5, 8, 14, 2, true), V_TCBD(EUL, 5, 8, 14, 2, true))
-DGLM_VARIANTS(EUL, 6, V_DMMA(EUL, 6, 8, 1, 6), V_SIMT(EUL, 6, 8, 7, 5),
+DGLM_VARIANTS(EUL, 6, sym_variant(6, 17), V_DMMA(EUL, 6, 8, 1, 6), V_SIMT(EUL, 6, 8, 7, 5),
               V_PIPEG(EUL, 6, 8, 1, false, 2, 2), V_PIPEG(EUL, 6, 8, 1, false, 2, 1),
               V_PM16G(EUL, 6, 8, 1, 2, 1, 2), V_PM16G(EUL, 6, 8, 1, 2, 2, 2),
               V_PM16G(EUL, 6, 8, 1, 2, 3, 2),

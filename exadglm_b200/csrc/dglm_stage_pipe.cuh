@@ -21,112 +21,6 @@
 // This header is included inside namespace dglm.
 #pragma once
 
-__device__ __forceinline__ unsigned smem_u32(const void *p) {
-  return (unsigned)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(unsigned long long *b, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long *b, unsigned tx) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)),
-               "r"(tx)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(unsigned long long *b) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long *b, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(b)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool mbar_test_wait(unsigned long long *b, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(b)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// bounded wait for the completion of the phase with the given parity.  With
-// the default bound the thread suspends in try_wait between checks; a
-// shortened bound (dglm_set_wait_limit) polls with the non-blocking
-// test_wait, so that the bound and not try_wait's own suspension time decides
-// when the wait gives up
-__device__ __forceinline__ bool mbar_wait(unsigned long long *b, unsigned parity,
-                                          long long limit = kWaitCycles) {
-  if (limit < kWaitCycles) {
-    const long long t0 = clock64();
-    while (!mbar_test_wait(b, parity))
-      if (clock64() - t0 > limit) return false;
-    return true;
-  }
-  if (mbar_try_wait(b, parity)) return true;
-  const long long t0 = clock64();
-  while (!mbar_try_wait(b, parity))
-    if (clock64() - t0 > limit) return false;
-  return true;
-}
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned bytes,
-                                         unsigned long long *bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-          "r"(smem_u32(dst)),
-      "l"(src), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
-}
-__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_arrive_noinc(unsigned long long *b) {
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(b))
-               : "memory");
-}
-__device__ __forceinline__ void consumer_sync(int nthreads) {
-  asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
-}
-// named barrier `id` over `nthreads` threads (consumer groups of the
-// ping-pong variants use ids 1 + 2g and 2 + 2g)
-__device__ __forceinline__ void group_sync(int id, int nthreads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-__device__ __forceinline__ bool group_all(bool v, int id, int nthreads) {
-  unsigned r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 p, %1, 0;\n\t"
-      "bar.red.and.pred q, %2, %3, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(r)
-      : "r"((unsigned)v), "r"(id), "r"(nthreads)
-      : "memory");
-  return r != 0;
-}
-// AND of a predicate over the consumer threads (named barrier 2)
-__device__ __forceinline__ bool consumer_all(bool v, int nthreads) {
-  unsigned r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 p, %1, 0;\n\t"
-      "bar.red.and.pred q, 2, %2, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(r)
-      : "r"((unsigned)v), "r"(nthreads)
-      : "memory");
-  return r != 0;
-}
-
 template <int PHYS, int N, int E_, int WN_, int WM_, bool ASMEM, int NG_ = 1, int PR_ = 0,
           int NB_ = 2, int PW_ = 1, int KSP_ = 1, bool FU_ = false, bool KG_ = false,
           int CPS_ = 1>
