@@ -215,8 +215,14 @@ struct StageVariant {
   cudaError_t (*launch)(const StageArgs &, cudaStream_t);
 };
 
-// Symmetry-adapted Euler stage (dglm_stage_sym.cu), orders 3..6.
-StageVariant sym_variant(int N, int fallback);
+// Symmetry-adapted stage (dglm_stage_sym.cu): Euler orders 3..6, advection 2..6.
+StageVariant sym_variant(int physics, int N, int fallback);
+// Flow records of the advection kernel (dglm_stage_sym_adv.cuh): doubles for K
+// elements, and their making from the uploaded mesh (legacy stream).
+size_t sym_flow_doubles(int N, int K);
+cudaError_t launch_sym_flow(int N, const double *image, const double *geo, const double *nrm,
+                            const double *fscale, const double *vel, const int *vmapP, long vs,
+                            long Kp, int K, double *flow);
 // Its operator image from A = [WDr WDs WDt -LIFT] (Np rows, row-major); false
 // when the operators or Fmask lack the symmetry of the reference tetrahedron.
 bool sym_operator_image(int N, const double *A, const int *Fmask, std::vector<double> &img);

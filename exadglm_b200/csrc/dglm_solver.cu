@@ -660,7 +660,7 @@ dglm_status dglm_upload_mesh(dglm_handle *h, const dglm_mesh_arrays *m) {
   cudaStreamSynchronize(h->stream);
   free_tape(h);   // the adjoint's operators and face pairing belong to the old mesh
   const auto H2D = cudaMemcpyHostToDevice;
-  h->op_symmetric = h->d.physics == DGLM_EULER && h->d.precision == DGLM_PREC_FP64 &&
+  h->op_symmetric = h->d.precision == DGLM_PREC_FP64 &&
                     sym_operator_image(h->d.N, h->Ahost.data(), m->Fmask, h->sym_image);
   choose_run_variant(h);
   drop_graphs(h);
@@ -679,6 +679,23 @@ dglm_status dglm_upload_mesh(dglm_handle *h, const dglm_mesh_arrays *m) {
     const double *v3[3] = {m->vx, m->vy, m->vz};
     for (int q = 0; q < 3 && e == cudaSuccess; q++)
       e = cudaMemcpy(h->vel + (size_t)q * h->vs, v3[q], sizeof(double) * K * Np, H2D);
+  }
+  if (e == cudaSuccess && h->d.physics == DGLM_ADVECTION && h->op_symmetric) {
+    // flow records of the symmetry-adapted advection kernel, whatever variant
+    // is selected (their operator image is uploaded for them alone)
+    if (!h->erec) {
+      dglm_status st = dalloc(h, &h->erec, sym_flow_doubles(h->d.N, h->d.K));
+      if (st != DGLM_OK) return st;
+    }
+    double *img = nullptr;
+    e = cudaMalloc(&img, sizeof(double) * h->sym_image.size());
+    if (e == cudaSuccess)
+      e = cudaMemcpy(img, h->sym_image.data(), sizeof(double) * h->sym_image.size(), H2D);
+    if (e == cudaSuccess)
+      e = launch_sym_flow(h->d.N, img, h->geo, h->nrm, h->fscale, h->vel, h->vmapP, h->vs, h->Kp,
+                          h->d.K, h->erec);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+    cudaFree(img);
   }
   if (e != cudaSuccess) return cuda_check(e, "dglm_upload_mesh");
   h->mesh_ready = true;
@@ -942,7 +959,7 @@ dglm_status dglm_stage(dglm_handle *h, int stage, double dt) {
   StageArgs a = stage_args(h, h->u[h->cur], h->u[h->cur ^ 1], stage);
   a.dt_override = dt;
   // the symmetry-adapted kernel leaves the wave speeds to the separate kernel
-  const bool sep = a.last_stage && h->vinfo.mode == MODE_SYM;
+  const bool sep = separate_maxv(h) && a.last_stage && h->vinfo.mode == MODE_SYM;
   if (sep) a.last_stage = 0;
   cudaError_t e = launch_stage_fp64(h->d.physics, h->d.N, h->run_variant, a, h->stream);
   if (e == cudaSuccess && sep)

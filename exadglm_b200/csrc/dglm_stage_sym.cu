@@ -13,6 +13,7 @@
 namespace dglm {
 
 #include "dglm_stage_sym.cuh"
+#include "dglm_stage_sym_adv.cuh"
 
 namespace {
 
@@ -327,6 +328,50 @@ StageVariant make_sym(int fallback) {
   return StageVariant{i, &launch_sym<N, NS, NG, NB>};
 }
 
+template <int N, int NW>
+cudaError_t launch_sym_adv(const StageArgs &a, cudaStream_t s) {
+  using C = SymAdvCfg<N, NW>;
+  auto k = stage_sym_adv_kernel<N, NW>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)C::SMEM);
+  if (e != cudaSuccess) return e;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (sms <= 0) sms = 148;
+  const int ntiles = (a.K + C::E - 1) / C::E;
+  k<<<ntiles < sms ? ntiles : sms, C::THREADS, C::SMEM, s>>>(a, ntiles);
+  return cudaGetLastError();
+}
+
+template <int N, int NW>
+StageVariant make_sym_adv(int fallback) {
+  using C = SymAdvCfg<N, NW>;
+  StageVariantInfo i{};
+  i.mode = MODE_SYM;
+  i.E = C::E;
+  i.threads = C::THREADS;
+  i.smem = C::SMEM;
+  i.bimg = 8 * C::S_A + 4 * ((C::Z::TABS + 1) / 2 * 2);
+  i.groups = NW;
+  i.R = 1;
+  i.ring = 2;
+  i.persistent = 1;
+  i.fallback = fallback;
+  return StageVariant{i, &launch_sym_adv<N, NW>};
+}
+
+template <int N>
+cudaError_t flow_launch(const double *image, const double *geo, const double *nrm,
+                        const double *fscale, const double *vel, const int *vmapP, long vs,
+                        long Kp, int K, double *flow) {
+  const int ntiles = (K + 7) / 8;
+  const long n = (long)ntiles * 32 * (SymSize<N>::KSV + SymSize<N>::KSF);
+  sym_flow_kernel<N><<<(unsigned)((n + 255) / 256), 256>>>(image, geo, nrm, fscale, vel, vmapP,
+                                                           vs, Kp, K, ntiles, flow);
+  return cudaGetLastError();
+}
+
 __global__ void element_record_kernel(const double *__restrict__ geo,
                                       const double *__restrict__ nrm,
                                       const double *__restrict__ fscale, long Kp, bool sym,
@@ -356,7 +401,21 @@ cudaError_t launch_element_records(const double *geo, const double *nrm, const d
   return cudaGetLastError();
 }
 
-StageVariant sym_variant(int N, int fallback) {
+StageVariant sym_variant(int physics, int N, int fallback) {
+  // Warps per CTA: what the registers allow, less where the shared memory they
+  // take is better left to L1 for the gathers (N=6, K=63,888: 8 warps 0.125 ms
+  // per stage, 12 warps 0.154; N=3, K=162,000: 24 0.057, 16 0.059, 12 0.063;
+  // N=5, K=93,750: 16 0.092, 12 0.097, 20 0.111).  Against the dense kernels:
+  // N=2, K=384,000 0.307 -> 0.080, N=3 0.097 -> 0.057, N=4, K=105,456 0.117 ->
+  // 0.061, N=5 0.236 -> 0.092 (58 % of the HBM copy rate for its bytes), N=6
+  // 0.254 -> 0.125.
+  if (physics == DGLM_ADVECTION) switch (N) {
+    case 2: return make_sym_adv<2, 16>(fallback);
+    case 3: return make_sym_adv<3, 24>(fallback);
+    case 4: return make_sym_adv<4, 16>(fallback);
+    case 5: return make_sym_adv<5, 16>(fallback);
+    default: return make_sym_adv<6, 8>(fallback);
+  }
   switch (N) {
     case 3: return make_sym<3, 1, 4, 8>(fallback);
     case 4: return make_sym<4, 1, 4, 6>(fallback);
@@ -365,12 +424,13 @@ StageVariant sym_variant(int N, int fallback) {
   }
 }
 
-#define SYM_ORDER(N, CALL)       \
+#define SYM_ORDER(N, ...)        \
   switch (N) {                   \
-    case 3: { constexpr int n = 3; CALL; break; } \
-    case 4: { constexpr int n = 4; CALL; break; } \
-    case 5: { constexpr int n = 5; CALL; break; } \
-    case 6: { constexpr int n = 6; CALL; break; } \
+    case 2: { constexpr int n = 2; __VA_ARGS__; break; } \
+    case 3: { constexpr int n = 3; __VA_ARGS__; break; } \
+    case 4: { constexpr int n = 4; __VA_ARGS__; break; } \
+    case 5: { constexpr int n = 5; __VA_ARGS__; break; } \
+    case 6: { constexpr int n = 6; __VA_ARGS__; break; } \
     default: break;              \
   }
 
@@ -378,6 +438,20 @@ bool sym_operator_image(int N, const double *A, const int *Fmask, std::vector<do
   bool ok = false;
   SYM_ORDER(N, ok = build_image<n>(A, Fmask, img))
   return ok;
+}
+
+size_t sym_flow_doubles(int N, int K) {
+  size_t per = 0;
+  SYM_ORDER(N, per = SymAdvCfg<n, 4>::FLOW)
+  return per * (((size_t)K + 7) / 8);
+}
+
+cudaError_t launch_sym_flow(int N, const double *image, const double *geo, const double *nrm,
+                            const double *fscale, const double *vel, const int *vmapP, long vs,
+                            long Kp, int K, double *flow) {
+  cudaError_t e = cudaErrorInvalidValue;
+  SYM_ORDER(N, e = flow_launch<n>(image, geo, nrm, fscale, vel, vmapP, vs, Kp, K, flow))
+  return e;
 }
 
 void sym_reorder_register(int N, long tiles, int nvar, long vs, const double *in, double *out,

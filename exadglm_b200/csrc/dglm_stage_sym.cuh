@@ -187,6 +187,39 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void *src, unsigned bytes
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 
+// chi_1..chi_3 values of this lane's slot of chi_0's m-tile m, column half h
+// (m is a literal after unrolling; the whole warp takes part).
+template <class C>
+__device__ __forceinline__ void sym_characters(const double (&acc)[C::MTT][2], int m, int h,
+                                               int row, int lane, double &y1, double &y2,
+                                               double &y3) {
+  constexpr int MT0 = C::MT0, MTB = C::MTB;
+  const int mb = m < MTB ? m : 0;
+  if constexpr (C::ALIGNED || C::N2 == 0) {
+    y1 = m < MTB ? acc[MT0 + mb][h] : 0.0;
+    y2 = m < MTB ? acc[MT0 + MTB + mb][h] : 0.0;
+    y3 = m < MTB ? acc[MT0 + 2 * MTB + mb][h] : 0.0;
+  } else {
+    // size-2 orbits: chi_1's rows are in chi_0's slots of involution 1; those
+    // of chi_2 and chi_3 sit in the same rows of their last tile
+    constexpr int ML = MTB - 1, RS = C::N4 - 8 * ML;   // first special row of that tile
+    static_assert(C::N4 + C::N2 == 8 * MTB && MT0 == MTB + 1, "layout of the size-2 rows");
+    if (m < MTB) {
+      const bool sp = m == ML && row >= RS;
+      y1 = acc[MT0 + mb][h];
+      y2 = sp ? 0.0 : acc[MT0 + MTB + mb][h];
+      y3 = sp ? 0.0 : acc[MT0 + 2 * MTB + mb][h];
+    } else {
+      const int src = (RS + (row < C::N2 ? row : row - C::N2)) * 4 + (lane & 3);
+      const double t2 = __shfl_sync(0xffffffffu, acc[MT0 + MTB + ML][h], src & 31);
+      const double t3 = __shfl_sync(0xffffffffu, acc[MT0 + 2 * MTB + ML][h], src & 31);
+      y1 = 0.0;
+      y2 = row < C::N2 ? t2 : 0.0;
+      y3 = row >= C::N2 && row < 2 * C::N2 ? t3 : 0.0;
+    }
+  }
+}
+
 // One warp's share of a tile's stage: variables [V0, V0 + NVW).
 template <class C, int V0, int NVW>
 struct SymWarp {
@@ -407,29 +440,7 @@ struct SymWarp {
       for (int h = 0; h < 2; h++) {
         const double y0 = acc[v][m][h];
         double y1, y2, y3;
-        if constexpr (C::ALIGNED || C::N2 == 0) {
-          y1 = m < MTB ? acc[v][mt0(1) + (m < MTB ? m : 0)][h] : 0.0;
-          y2 = m < MTB ? acc[v][mt0(2) + (m < MTB ? m : 0)][h] : 0.0;
-          y3 = m < MTB ? acc[v][mt0(3) + (m < MTB ? m : 0)][h] : 0.0;
-        } else {
-          // size-2 orbits: chi_1's rows are in chi_0's slots of involution 1;
-          // those of chi_2 and chi_3 sit in the same rows of their last tile
-          constexpr int ML = MTB - 1, RS = C::N4 - 8 * ML;   // first special row of that tile
-          static_assert(C::N4 + C::N2 == 8 * MTB && MT0 == MTB + 1, "layout of the size-2 rows");
-          if (m < MTB) {
-            const bool sp = m == ML && row >= RS;
-            y1 = acc[v][mt0(1) + (m < MTB ? m : 0)][h];
-            y2 = sp ? 0.0 : acc[v][mt0(2) + (m < MTB ? m : 0)][h];
-            y3 = sp ? 0.0 : acc[v][mt0(3) + (m < MTB ? m : 0)][h];
-          } else {
-            const int src = (RS + (row < C::N2 ? row : row - C::N2)) * 4 + (lane & 3);
-            const double t2 = __shfl_sync(0xffffffffu, acc[v][mt0(2) + ML][h], src & 31);
-            const double t3 = __shfl_sync(0xffffffffu, acc[v][mt0(3) + ML][h], src & 31);
-            y1 = 0.0;
-            y2 = row < C::N2 ? t2 : 0.0;
-            y3 = row >= C::N2 && row < 2 * C::N2 ? t3 : 0.0;
-          }
-        }
+        sym_characters<C>(acc[v], m, h, row, lane, y1, y2, y3);
         const double s01 = y0 + y1, d01 = y0 - y1, s23 = y2 + y3, d23 = y2 - y3;
         double *const u = h ? u1 : u0;
         const double *const o = un[m][h];

@@ -1,4 +1,4 @@
-"""The symmetry-adapted FP64 Euler kernel (variants "pipe-dmma-sym").
+"""The symmetry-adapted FP64 kernels (variants "pipe-dmma-sym").
 
 On the CPU: the decomposition it computes (projections on the characters of
 the four vertex permutations, restated here in numpy from its definition)
@@ -12,8 +12,6 @@ remainders, meshes smaller than the grid and several times a block's ring of
 buffers; operators without the symmetry, which run on the variant's fallback;
 and a change of variant in the middle of a step, where the register changes
 its order."""
-import itertools
-
 import numpy as np
 import pytest
 
@@ -30,13 +28,21 @@ def rel(a, b):
     return float(np.linalg.norm(np.ravel(a) - np.ravel(b)) / np.linalg.norm(np.ravel(b)))
 
 
-def euler(N, cells):
+PHYS = [("euler", N) for N in (3, 4, 5, 6)] + [("advection", N) for N in (2, 3, 4, 5, 6)]
+
+
+def make(phys, N, cells):
     mesh = Mesh3D(N, UniformBox(*(c + 1 for c in cells)), high_order=False)
-    return P.euler_sine(N=N, noise=1e-3, seed=N, mesh=mesh)
+    if phys == "euler":
+        return P.euler_sine(N=N, noise=1e-3, seed=N, mesh=mesh)
+    prob = P.advection_gaussian(N=N, width2=0.05, mesh=mesh)
+    # a velocity of its own at every node (tau and the fluxes take it as it is)
+    prob.vel = prob.vel * (1 + 0.1 * np.random.default_rng(N).standard_normal(prob.vel.shape))
+    return prob
 
 
-def sym_variant(N):
-    return [v for v, d in variants("euler", N, "fp64") if d.startswith("pipe-dmma-sym")][0]
+def sym_variant(phys, N):
+    return [v for v, d in variants(phys, N, "fp64") if d.startswith("pipe-dmma-sym")][0]
 
 
 @pytest.mark.parametrize("N", range(1, 9))
@@ -75,14 +81,13 @@ def test_decomposition_equals_dense_operators(N):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("N,cells", [
-    *itertools.product((3, 4, 5, 6), ((2, 2, 2), (2, 3, 3), (5, 3, 3), (3, 3, 3))),
-    (3, (16, 12, 12)), (4, (12, 12, 12)), (5, (11, 9, 7)), (6, (9, 9, 7))])
-def test_sizes_match_oracle(N, cells):
+@pytest.mark.parametrize("phys,N", PHYS)
+@pytest.mark.parametrize("cells", [(2, 2, 2), (2, 3, 3), (5, 3, 3), (3, 3, 3), (11, 9, 10)])
+def test_sizes_match_oracle(phys, N, cells):
     """K = 48, 108, 270, 162 (whole tiles, remainders of 4, 6 and 2 elements)
-    and meshes of several tiles per group."""
-    prob = euler(N, cells)
-    s = Solver(prob, variant=sym_variant(N))
+    and 5,940, several tiles per group."""
+    prob = make(phys, N, cells)
+    s = Solver(prob, variant=sym_variant(phys, N))
     s.step(2)
     s.sync()
     uo, _, clk, _ = oracle.Oracle(prob).run(2)
@@ -92,15 +97,15 @@ def test_sizes_match_oracle(N, cells):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("N", (3, 4, 5, 6))
-def test_operators_without_the_symmetry(N):
-    prob = euler(N, (3, 3, 3))
+@pytest.mark.parametrize("phys,N", PHYS)
+def test_operators_without_the_symmetry(phys, N):
+    prob = make(phys, N, (3, 3, 3))
     arr = {k: np.array(v, copy=True) for k, v in prob.datain_arrays().items()}
     arr["WDs"] = arr["WDs"] * (1 + 1e-9 * np.random.default_rng(0).standard_normal(
         np.shape(arr["WDs"])))
     prob.datain_arrays = lambda: arr
-    s = Solver(prob, variant=sym_variant(N))
-    assert s.variant() == sym_variant(N)
+    s = Solver(prob, variant=sym_variant(phys, N))
+    assert s.variant() == sym_variant(phys, N)
     s.step(3)
     s.sync()
     assert rel(s.get_state(), oracle.Oracle(prob).run(3)[0]) < TOL
@@ -108,18 +113,18 @@ def test_operators_without_the_symmetry(N):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("N", (3, 4, 5, 6))
-def test_variant_change_between_stages(N):
+@pytest.mark.parametrize("phys,N", PHYS)
+def test_variant_change_between_stages(phys, N):
     """The five stages of a step on two variants in turn give the state of the
     step on one."""
-    prob = euler(N, (3, 3, 3))
-    other = [v for v, d in variants("euler", N, "fp64") if not d.startswith("pipe-dmma-sym")][0]
-    one = Solver(prob, variant=sym_variant(N))
+    prob = make(phys, N, (3, 3, 3))
+    other = [v for v, d in variants(phys, N, "fp64") if not d.startswith("pipe-dmma-sym")][0]
+    one = Solver(prob, variant=sym_variant(phys, N))
     for st in range(5):
         one.stage(st, 1e-3)
-    two = Solver(prob, variant=sym_variant(N))
+    two = Solver(prob, variant=sym_variant(phys, N))
     for st in range(5):
-        two.set_variant(other if st % 2 else sym_variant(N))
+        two.set_variant(other if st % 2 else sym_variant(phys, N))
         two.stage(st, 1e-3)
     assert rel(two.get_state(), one.get_state()) < 1e-14
     one.close()
