@@ -10,6 +10,12 @@
 // function compiled for the tile's order -- one launch covers every order.
 // The list is sorted by order, largest first, so each CTA gets a similar mix.
 //
+// Operators with the symmetry of the reference tetrahedron (every symmetric
+// node set's) run on batch_sym_kernel: tiles of 8 elements, a warp per tile,
+// the symmetry-adapted advection tile of dglm_stage_sym_adv.cuh.  The tile
+// list is sorted by order; each CTA takes one stretch of it, cut by cost, and
+// loads an order's operator once per stretch.  Otherwise batch_stage_kernel:
+//
 // Per tile (advection, one variable): stage u and the tile's metrics and
 // face data in shared memory; volume fluxes v u combined with the metrics;
 // contraction with [WDr WDs WDt] on the FP64 tensor cores (m8n8k4, the
@@ -29,10 +35,12 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "dglm_common.cuh"
 #include "dglm_handle.cuh"
+#include "dglm_sym.cuh"
 
 namespace dglm {
 
@@ -298,6 +306,195 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_stage_kernel(const Bat
   }
 }
 
+// ---------------------------------------------------------------------------
+// symmetry-adapted path
+// ---------------------------------------------------------------------------
+
+struct BatchSymArgs {
+  const BatchTile *tiles;     // sorted by order, largest first
+  int begin[8];               // tiles of order N: [begin[N], begin[N - 1])
+  const int *cut;             // gridDim.x + 1: the CTAs' stretches of the tile list
+  const BatchInst *inst;
+  const BatchScalars *sc;
+  const double *image[kMaxOrder + 1];   // operator images per order
+  const double *rec;          // per element: kSymRec flux weights
+  const int *nb[kMaxOrder + 1];         // per tile of an order: neighbour nodes, lane order
+  const double *u_in;
+  double *u_out, *kreg;
+  double rka, rkb;
+  int *err;                   // set when a bounded wait expired
+};
+
+// Per element: (grad r_a + sum_b grad r_b) . v (a = 1..3), Fscale n . v / 2 and
+// Fscale tau / 2 of the four faces by label, one pad.
+constexpr int kSymRec = 12;
+constexpr int kSymWarps = 12;
+// warps that take tiles of order N (N=6: the state buffers of eight leave L1
+// room for the gathers)
+template <int N>
+constexpr int sym_warps() {
+  return N == 6 ? 8 : kSymWarps;
+}
+template <int N>
+using BSC = SymAdvCfg<N, sym_warps<N>()>;
+constexpr size_t kBatchSymSmem =
+    cmax(cmax(cmax(BSC<2>::SMEM, BSC<3>::SMEM), cmax(BSC<4>::SMEM, BSC<5>::SMEM)),
+         BSC<6>::SMEM) + 16 * kSymWarps;
+// Cost of a tile of order N (measured ns of a device's stage per tile), the
+// weight by which the stretches are cut.
+constexpr double kSymCost[7] = {0, 0, 1.7, 2.9, 4.6, 8.3, 15.7};
+
+// Tiles [lo, hi) of order N by this CTA.  it: buffer uses of the warp so far.
+template <int N>
+__device__ __forceinline__ bool batch_sym_tiles(const BatchSymArgs &a, int lo, int hi,
+                                                double *smem, unsigned long long *full,
+                                                int &it) {
+  using C = BSC<N>;
+  constexpr int NW = sym_warps<N>(), Np = C::Np, P4 = 32 * C::KSF;
+  double *sBuf = smem + C::S_A;
+  int *tabs = reinterpret_cast<int *>(sBuf + NW * 2 * C::S_U);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const SymAdvOp op = sym_adv_operator<C>(a.image[N], smem, tabs, tid, 32 * kSymWarps);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncthreads();
+  bool ok = true;
+  if (warp < NW && lo + warp < hi) {
+    double *buf = sBuf + warp * 2 * C::S_U;
+    auto fetch = [&](int ti, int b) {   // lane 0
+      const BatchTile t = a.tiles[ti];
+      mbar_arrive_expect_tx(&full[b], 8u * C::S_U);
+      bulk_g2s(buf + b * C::S_U, a.u_in + a.inst[t.inst].node_off + (long)t.e0 * Np,
+               8u * C::S_U, &full[b]);
+    };
+    if (lane == 0) fetch(lo + warp, it & 1);
+    for (int ti = lo + warp; ti < hi; ti += NW, it++) {
+      const int b = it & 1;
+      const BatchTile t = a.tiles[ti];
+      const BatchInst &I = a.inst[t.inst];
+      const long node0 = I.node_off + (long)t.e0 * Np;
+      double *u = buf + b * C::S_U;
+      FlowConstant fl;
+      double s[4];
+      {
+        // elements past the instance's last: zero weights on a zero state
+        const int el = C::elem(lane >> 2);
+        double2 q[kSymRec / 2];
+#pragma unroll
+        for (int i = 0; i < kSymRec / 2; i++)
+          q[i] = el < t.ne ? __ldg(reinterpret_cast<const double2 *>(
+                                 a.rec + (I.elem_off + t.e0 + el) * kSymRec) + i)
+                           : make_double2(0.0, 0.0);
+        fl.va[0] = q[0].x, fl.va[1] = q[0].y, fl.va[2] = q[1].x;
+        fl.wf[0] = q[1].y, fl.wf[1] = q[2].x, fl.wf[2] = q[2].y, fl.wf[3] = q[3].x;
+        s[0] = q[3].y, s[1] = q[4].x, s[2] = q[4].y, s[3] = q[5].x;
+      }
+      ok = sym_adv_tile<C>(
+          op, u, fl,
+          reinterpret_cast<const int4 *>(a.nb[N]) + (long)(ti - a.begin[N]) * P4 + lane,
+          a.u_in + I.node_off, s, a.kreg + node0, a.sc[t.inst].dt, a.rka, a.rkb, a.rka != 0.0,
+          false, lane,
+          [&]() { return __all_sync(0xffffffffu, mbar_wait(&full[b], (it >> 1) & 1)) != 0; },
+          [&]() {
+            // the next tile's state, once the previous tile's store has read its buffer
+            if (lane == 0 && ti + NW < hi) {
+              bulk_wait_read();
+              fetch(ti + NW, b ^ 1);
+            }
+          });
+      if (!ok) {
+        if (lane == 0) *a.err = 1;
+        break;
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) {
+        bulk_s2g(a.u_out + node0, u, 8u * C::S_U);
+        bulk_commit();
+      }
+    }
+    if (lane == 0) bulk_wait_all();
+  }
+  // the shared memory of this stretch is free
+  return __syncthreads_and(ok) != 0;
+}
+
+__global__ void __launch_bounds__(32 * kSymWarps, 1) batch_sym_kernel(const BatchSymArgs a) {
+  extern __shared__ __align__(16) double smem[];
+  // the warps' barriers sit behind the largest order's layout
+  unsigned long long *full = reinterpret_cast<unsigned long long *>(
+      reinterpret_cast<char *>(smem) + kBatchSymSmem - 16 * kSymWarps) + 2 * (threadIdx.x >> 5);
+  if ((threadIdx.x & 31) == 0) {
+    mbar_init(&full[0], 1);
+    mbar_init(&full[1], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  const int first = a.cut[blockIdx.x], last = a.cut[blockIdx.x + 1];
+  int it = 0;
+  bool ok = true;
+  auto stretch = [&](int N, int &lo, int &hi) {
+    lo = max(first, a.begin[N]);
+    hi = min(last, a.begin[N - 1]);
+    return ok && lo < hi;
+  };
+  int lo, hi;
+  if (stretch(6, lo, hi)) ok = batch_sym_tiles<6>(a, lo, hi, smem, full, it);
+  if (stretch(5, lo, hi)) ok = batch_sym_tiles<5>(a, lo, hi, smem, full, it);
+  if (stretch(4, lo, hi)) ok = batch_sym_tiles<4>(a, lo, hi, smem, full, it);
+  if (stretch(3, lo, hi)) ok = batch_sym_tiles<3>(a, lo, hi, smem, full, it);
+  if (stretch(2, lo, hi)) ok = batch_sym_tiles<2>(a, lo, hi, smem, full, it);
+}
+
+// Neighbour nodes of the tiles of order N in lane order (instance-local).
+template <int N>
+__global__ void batch_neighbour_kernel(const double *__restrict__ image,
+                                       const BatchTile *__restrict__ tiles, int ntiles,
+                                       const BatchInst *__restrict__ inst,
+                                       const int *__restrict__ vmapP, int *__restrict__ nb) {
+  using C = BSC<N>;
+  constexpr int P4 = 32 * C::KSF;
+  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (i >= (long)ntiles * P4) return;
+  const int ti = (int)(i / P4), p = (int)(i % P4), f = p / 32, lane = p % 32;
+  const BatchTile t = tiles[ti];
+  const int el = C::elem(lane >> 2), j = min(f * 4 + (lane & 3), C::Nfp - 1);
+  const int *tab = reinterpret_cast<const int *>(image + C::S_A) + C::T_VOL + j * 4;
+  for (int v = 0; v < 4; v++)
+    nb[i * 4 + v] = el < t.ne ? vmapP[inst[t.inst].fp_off + (long)(t.e0 + el) * C::NFF + (tab[v] >> 16)]
+                              : 0;
+}
+
+// Flux weights of every element of every instance (blockIdx.y).
+__global__ void batch_record_kernel(const BatchInst *__restrict__ inst,
+                                    const int *const *__restrict__ labels,
+                                    const double *__restrict__ geo,
+                                    const double *__restrict__ nrm,
+                                    const double *__restrict__ fscale, long gs,
+                                    double *__restrict__ rec) {
+  const BatchInst I = inst[blockIdx.y];
+  const int *face_of = labels[I.N];
+  const double v[3] = {I.vx, I.vy, I.vz};
+  for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < I.K;
+       k += (long)gridDim.x * blockDim.x) {
+    const long e = I.elem_off + k;
+    double *r = rec + e * kSymRec;
+    for (int d = 0; d < 3; d++) {
+      double x = 0.0;
+      for (int q = 0; q < 3; q++)
+        x += (geo[(3 * d + q) * gs + e] +
+              (geo[q * gs + e] + geo[(3 + q) * gs + e] + geo[(6 + q) * gs + e])) * v[q];
+      r[d] = x;
+    }
+    for (int l = 0; l < 4; l++) {
+      const long f = 4 * e + face_of[l];
+      double vn = 0.0;
+      for (int q = 0; q < 3; q++) vn += nrm[4 * q * gs + f] * v[q];
+      r[3 + l] = 0.5 * fscale[f] * vn;
+      r[7 + l] = 0.5 * fscale[f] * I.tau;
+    }
+    r[11] = 0.0;
+  }
+}
+
 // Per-instance max of |v| Fscale over its faces (calc_maxv + calc_dt of the
 // reference with a frozen velocity), one block per instance.
 __global__ void batch_wavespeed_kernel(const BatchInst *inst, const double *fscale,
@@ -377,6 +574,9 @@ struct dglm_batch {
   double *u[2] = {nullptr, nullptr};
   int cur = 0, ntiles = 0, grid = 0;
   std::vector<BatchInst> hinst;
+  bool sym = false;                 // all orders on the symmetry-adapted path
+  BatchSymArgs sargs{};
+  int *err = nullptr;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   long launches = 0;
 };
@@ -464,8 +664,18 @@ cudaError_t issue_batch_step(dglm_batch *b, int cur, cudaStream_t s) {
   batch_step_begin_kernel<<<nb, tb, 0, s>>>(n, b->inst, b->d.cfl, b->d.tmax, b->sc);
   cudaError_t e = cudaGetLastError();
   for (int st = 0; st < 5 && e == cudaSuccess; st++) {
-    BatchArgs a = b->args;
     const int in = (cur + st) & 1;
+    if (b->sym) {
+      BatchSymArgs q = b->sargs;
+      q.u_in = b->u[in];
+      q.u_out = b->u[in ^ 1];
+      q.rka = RKA[st];
+      q.rkb = RKB[st];
+      batch_sym_kernel<<<b->grid, 32 * kSymWarps, kBatchSymSmem, s>>>(q);
+      e = cudaGetLastError();
+      continue;
+    }
+    BatchArgs a = b->args;
     a.u_in = b->u[in];
     a.u_out = b->u[in ^ 1];
     a.rka = RKA[st];
@@ -478,6 +688,115 @@ cudaError_t issue_batch_step(dglm_batch *b, int cur, cudaStream_t s) {
     e = cudaGetLastError();
   }
   return e;
+}
+
+template <int N>
+std::pair<size_t, int> label_offset() {
+  using Z = SymSize<N>;
+  return {(size_t)Z::S_A, Z::T_VOL + Z::T_FACE + Z::T_OUT};
+}
+// where an operator image holds its face labels: (doubles, then ints)
+std::pair<size_t, int> sym_label_offset(int N) {
+  switch (N) {
+    case 2: return label_offset<2>();
+    case 3: return label_offset<3>();
+    case 4: return label_offset<4>();
+    case 5: return label_offset<5>();
+    default: return label_offset<6>();
+  }
+}
+// ints of a tile's neighbour list
+size_t sym_neighbour_ints(int N) { return (size_t)128 * ((nfp_of(N) + 3) / 4); }
+
+template <int N>
+cudaError_t launch_neighbours(dglm_batch *b, int begin, int ntiles, const int *vmapP, int *nb) {
+  const long n = (long)ntiles * 32 * BSC<N>::KSF;
+  batch_neighbour_kernel<N><<<(unsigned)((n + 255) / 256), 256>>>(
+      b->sargs.image[N], b->tiles + begin, ntiles, b->inst, vmapP, nb);
+  return cudaGetLastError();
+}
+
+// Operator images, flux weights, neighbour lists and the cut of the tile list
+// for the symmetry-adapted path.
+dglm_status finalize_sym(dglm_batch *b, const std::vector<BatchTile> &tiles,
+                         const std::vector<double> *image, const double *geo, const double *nrm,
+                         const double *fscale, long gs, const int *vmapP, double *kreg,
+                         long elems) {
+  BatchSymArgs &q = b->sargs;
+  q = BatchSymArgs{};
+  int count[kMaxOrder + 1] = {};
+  for (const BatchTile &t : tiles) count[t.N]++;
+  q.begin[7] = q.begin[6] = 0;
+  for (int N = 6; N >= 1; N--) q.begin[N - 1] = q.begin[N] + (N >= 2 ? count[N] : 0);
+  int sms = 0;
+  cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->dev);
+  if (e != cudaSuccess) return cuda_check(e, "dglm_batch_finalize");
+  b->grid = std::max(1, std::min((int)tiles.size(), sms));
+  // stretches of equal cost
+  double total = 0;
+  for (const BatchTile &t : tiles) total += kSymCost[t.N];
+  std::vector<int> cut(b->grid + 1, (int)tiles.size());
+  double sum = 0;
+  int c = 0;
+  for (int i = 0; i < (int)tiles.size() && c < b->grid; i++) {
+    while (c < b->grid && sum >= total * c / b->grid) cut[c++] = i;
+    sum += kSymCost[tiles[i].N];
+  }
+  double *rec = nullptr;
+  int *dcut = nullptr, *lab = nullptr;
+  const int **labels = nullptr;
+  dglm_status st = balloc(b, &rec, (size_t)elems * kSymRec);
+  if (st == DGLM_OK) st = balloc(b, &dcut, cut.size());
+  if (st == DGLM_OK) st = balloc(b, &lab, (size_t)4 * (kMaxOrder + 1));
+  if (st == DGLM_OK) st = balloc(b, &labels, (size_t)kMaxOrder + 1);
+  if (st == DGLM_OK) st = balloc(b, &b->err, 1);
+  if (st != DGLM_OK) return st;
+  const auto H2D = cudaMemcpyHostToDevice;
+  e = cudaMemcpy(dcut, cut.data(), sizeof(int) * cut.size(), H2D);
+  if (e == cudaSuccess) e = cudaMemset(b->err, 0, sizeof(int));
+  std::vector<const int *> hl(kMaxOrder + 1, nullptr);
+  for (int N = 2; N <= 6 && e == cudaSuccess; N++) {
+    if (image[N].empty()) continue;
+    double *img = nullptr;
+    int *nb = nullptr;
+    st = balloc(b, &img, image[N].size());
+    if (st == DGLM_OK) st = balloc(b, &nb, sym_neighbour_ints(N) * count[N]);
+    if (st != DGLM_OK) return st;
+    e = cudaMemcpy(img, image[N].data(), sizeof(double) * image[N].size(), H2D);
+    q.image[N] = img;
+    q.nb[N] = nb;
+    // the face labels sit behind the image's tables
+    hl[N] = reinterpret_cast<const int *>(img + sym_label_offset(N).first) +
+            sym_label_offset(N).second;
+    if (e != cudaSuccess) break;
+    switch (N) {
+      case 2: e = launch_neighbours<2>(b, q.begin[2], count[2], vmapP, nb); break;
+      case 3: e = launch_neighbours<3>(b, q.begin[3], count[3], vmapP, nb); break;
+      case 4: e = launch_neighbours<4>(b, q.begin[4], count[4], vmapP, nb); break;
+      case 5: e = launch_neighbours<5>(b, q.begin[5], count[5], vmapP, nb); break;
+      default: e = launch_neighbours<6>(b, q.begin[6], count[6], vmapP, nb); break;
+    }
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(labels, hl.data(), sizeof(int *) * hl.size(), H2D);
+  const int ninst = (int)b->hinst.size();
+  for (int i = 0; i < ninst && e == cudaSuccess; i += 65535) {
+    const int m = std::min(65535, ninst - i);
+    batch_record_kernel<<<dim3(16, m), 128>>>(b->inst + i, labels, geo, nrm, fscale, gs, rec);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(batch_sym_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kBatchSymSmem);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+  if (e != cudaSuccess) return cuda_check(e, "dglm_batch_finalize");
+  q.tiles = b->tiles;
+  q.cut = dcut;
+  q.inst = b->inst;
+  q.sc = b->sc;
+  q.rec = rec;
+  q.kreg = kreg;
+  q.err = b->err;
+  return DGLM_OK;
 }
 
 }  // namespace
@@ -582,6 +901,11 @@ dglm_status dglm_batch_finalize(dglm_batch *b) {
   if (b->host.empty()) return set_error(DGLM_ERR_STATE, "dglm_batch_finalize: no instances");
   DeviceGuard g(b->dev);
   const int n = (int)b->host.size();
+  std::vector<double> image[kMaxOrder + 1];
+  b->sym = true;
+  for (int N = 2; N <= 6; N++)
+    if (!b->Ahost[N].empty())
+      b->sym = b->sym && sym_operator_image(N, b->Ahost[N].data(), b->Fm[N].data(), image[N]);
   long nodes = 0, elems = 0, fps = 0;
   b->hinst.resize(n);
   for (int i = 0; i < n; i++) {
@@ -599,7 +923,8 @@ dglm_status dglm_batch_finalize(dglm_batch *b) {
     // update_tau with maxv = |v| on both sides (advec_dglm.cpp)
     const double mv = std::sqrt(I.vx * I.vx + I.vy * I.vy + I.vz * I.vz);
     I.tau = 0.25 * (mv + mv) * b->d.tau_scale;
-    nodes += ((long)H.K * Np + 31) / 32 * 32;
+    // whole tiles of 8 elements (their padding is zero and stays zero)
+    nodes += ((long)H.K + 7) / 8 * 8 * Np;
     elems += H.K;
     fps += (long)H.K * NFF;
   }
@@ -609,7 +934,7 @@ dglm_status dglm_batch_finalize(dglm_batch *b) {
   for (int N = 6; N >= 2; N--)
     for (int i = 0; i < n; i++) {
       if (b->host[i].N != N) continue;
-      const int E = tile_elems(N);
+      const int E = b->sym ? 8 : tile_elems(N);
       for (int e0 = 0; e0 < b->host[i].K; e0 += E)
         tiles.push_back(BatchTile{i, e0, std::min(E, b->host[i].K - e0), N});
     }
@@ -661,7 +986,7 @@ dglm_status dglm_batch_finalize(dglm_batch *b) {
   BatchArgs &a = b->args;
   a = BatchArgs{};
   for (int N = 2; N <= 6 && e == cudaSuccess; N++) {
-    if (b->Ahost[N].empty()) continue;
+    if (b->sym || b->Ahost[N].empty()) continue;
     std::vector<double> fr = fragments_for(N, b->Ahost[N]);
     double *dops = nullptr;
     int *dfm = nullptr;
@@ -684,6 +1009,10 @@ dglm_status dglm_batch_finalize(dglm_batch *b) {
   a.gs = gs;
   a.vmapP = dvm;
   a.kreg = dk;
+  if (b->sym) {
+    st = finalize_sym(b, tiles, image, dgeo, dnrm, dfs, gs, dvm, dk, elems);
+    if (st != DGLM_OK) return st;
+  }
   e = cudaFuncSetAttribute(batch_stage_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)kBatchSmem);
   int per_sm = 0, sms = 0;
@@ -692,7 +1021,7 @@ dglm_status dglm_batch_finalize(dglm_batch *b) {
                                                       kBatchThreads, kBatchSmem);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->dev);
   if (e != cudaSuccess) return cuda_check(e, "dglm_batch_finalize");
-  b->grid = std::max(1, std::min(b->ntiles, std::max(per_sm, 1) * sms));
+  if (!b->sym) b->grid = std::max(1, std::min(b->ntiles, std::max(per_sm, 1) * sms));
   batch_wavespeed_kernel<<<n, 256, 0, b->stream>>>(b->inst, dfs, b->sc);
   e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
@@ -743,7 +1072,14 @@ dglm_status dglm_batch_step(dglm_batch *b, int nsteps) {
 dglm_status dglm_batch_sync(dglm_batch *b) {
   if (!b) return set_error(DGLM_ERR_INVALID, "dglm_batch_sync: NULL batch");
   DeviceGuard g(b->dev);
-  return cuda_check(cudaStreamSynchronize(b->stream), "dglm_batch_sync");
+  cudaError_t e = cudaStreamSynchronize(b->stream);
+  int err = 0;
+  if (e == cudaSuccess && b->err)
+    e = cudaMemcpy(&err, b->err, sizeof(int), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess && err)
+    return set_error(DGLM_ERR_CUDA, "dglm_batch_sync: a bounded wait in the stage kernel expired; "
+                                    "results are invalid");
+  return cuda_check(e, "dglm_batch_sync");
 }
 
 int dglm_batch_count(dglm_batch *b) {

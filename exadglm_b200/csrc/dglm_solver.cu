@@ -682,20 +682,23 @@ dglm_status dglm_upload_mesh(dglm_handle *h, const dglm_mesh_arrays *m) {
   }
   if (e == cudaSuccess && h->d.physics == DGLM_ADVECTION && h->op_symmetric) {
     // flow records of the symmetry-adapted advection kernel, whatever variant
-    // is selected (their operator image is uploaded for them alone)
+    // is selected
     if (!h->erec) {
       dglm_status st = dalloc(h, &h->erec, sym_flow_doubles(h->d.N, h->d.K));
       if (st != DGLM_OK) return st;
     }
-    double *img = nullptr;
-    e = cudaMalloc(&img, sizeof(double) * h->sym_image.size());
+    // (AT holds the operator image unless another variant is selected)
+    const bool other = h->vinfo.mode != MODE_SYM;
+    if (other)
+      e = cudaMemcpy(h->AT, h->sym_image.data(), sizeof(double) * h->sym_image.size(), H2D);
     if (e == cudaSuccess)
-      e = cudaMemcpy(img, h->sym_image.data(), sizeof(double) * h->sym_image.size(), H2D);
-    if (e == cudaSuccess)
-      e = launch_sym_flow(h->d.N, img, h->geo, h->nrm, h->fscale, h->vel, h->vmapP, h->vs, h->Kp,
-                          h->d.K, h->erec);
+      e = launch_sym_flow(h->d.N, h->AT, h->geo, h->nrm, h->fscale, h->vel, h->vmapP, h->vs,
+                          h->Kp, h->d.K, h->erec);
     if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
-    cudaFree(img);
+    if (e == cudaSuccess && other) {
+      os = upload_operator_layout(h);
+      if (os != DGLM_OK) return os;
+    }
   }
   if (e != cudaSuccess) return cuda_check(e, "dglm_upload_mesh");
   h->mesh_ready = true;

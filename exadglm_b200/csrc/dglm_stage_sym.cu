@@ -7,13 +7,9 @@
 #include <cstring>
 #include <vector>
 
-#include "dglm_common.cuh"
-#include "dglm_ptx.cuh"
+#include "dglm_sym.cuh"
 
 namespace dglm {
-
-#include "dglm_stage_sym.cuh"
-#include "dglm_stage_sym_adv.cuh"
 
 namespace {
 

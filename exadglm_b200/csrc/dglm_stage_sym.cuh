@@ -1,5 +1,5 @@
 // FP64 Euler stage kernel on symmetry-adapted operators (included by
-// dglm_stage_sym.cu).
+// dglm_sym.cuh).
 //
 // The nodes of the reference tetrahedron are symmetric under the four vertex
 // permutations V4 = {id, (01)(23), (02)(13), (03)(12)}.  With the barycentric

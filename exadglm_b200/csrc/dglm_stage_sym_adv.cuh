@@ -1,5 +1,5 @@
 // FP64 advection stage on the symmetry-adapted operators of
-// dglm_stage_sym.cuh (included by dglm_stage_sym.cu).
+// dglm_stage_sym.cuh (included by dglm_sym.cuh).
 //
 // The fluxes of linear advection are the state times fixed numbers, so the
 // mesh upload forms those numbers once, in the order in which the kernel's
@@ -38,59 +38,69 @@ struct SymAdvCfg : SymSize<N> {
   static_assert(S_U % 2 == 0, "16-byte aligned copies");
 };
 
-template <int N, int NW>
-__global__ void __launch_bounds__(32 * NW, 1)
-    stage_sym_adv_kernel(const StageArgs a, int ntiles) {
-  using C = SymAdvCfg<N, NW>;
+// Flux weights of a tile, read from its flow record (single meshes), or the
+// lane's element's own for a velocity that is constant (batches).
+struct FlowRecord {
+  const double *V, *W;   // at the lane
+  __device__ __forceinline__ double vol(int ks, int d) const {
+    return __ldg(V + ks * 96 + 32 * d);
+  }
+  __device__ __forceinline__ double face(int f, int v) const {
+    return __ldg(W + f * 128 + 32 * v);
+  }
+};
+struct FlowConstant {
+  double va[3], wf[4];
+  __device__ __forceinline__ double vol(int, int d) const { return va[d]; }
+  __device__ __forceinline__ double face(int, int v) const { return wf[v]; }
+};
+
+// The operator image in shared memory: fragments and tables.
+struct SymAdvOp {
+  const double *A;
+  const int *tvol;       // nodes of the three images, 10 bits each
+  const int4 *tface, *tout;
+};
+// Copies it there (all threads of the block; the caller synchronises).
+template <class C>
+__device__ __forceinline__ SymAdvOp sym_adv_operator(const double *image, double *sA, int *tabs,
+                                                     int tid, int nt) {
+  const double2 *src = reinterpret_cast<const double2 *>(image);
+  double2 *dst = reinterpret_cast<double2 *>(sA);
+  for (int i = tid; i < C::S_A / 2; i += nt) dst[i] = __ldg(src + i);
+  const int *ts = reinterpret_cast<const int *>(image + C::S_A);
+  // volume entries with the images' nodes in place of the shuffle lanes
+  for (int i = tid; i < C::KSV * 4; i += nt) {
+    const int q = i & ~3, x = __ldg(ts + i);
+    tabs[i] = (__ldg(ts + (q | ((x >> 16) & 3))) & 0x3ff) |
+              (__ldg(ts + (q | ((x >> 18) & 3))) & 0x3ff) << 10 |
+              (__ldg(ts + (q | ((x >> 20) & 3))) & 0x3ff) << 20;
+  }
+  for (int i = tid; i < C::T_FACE + C::T_OUT; i += nt)
+    tabs[C::KSV * 4 + i] = __ldg(ts + C::T_VOL + i);
+  const int4 *tface = reinterpret_cast<const int4 *>(tabs + C::KSV * 4);
+  return SymAdvOp{sA, tabs, tface, tface + C::T_FACE / 4};
+}
+
+// One tile by one warp, in its state buffer u: returns false when the wait
+// for the buffer expired.  P: the tile's neighbour nodes at the lane, counted
+// from ubase; s: Fscale tau / 2 of the lane's element's faces by label; kt: the
+// tile's register.  wait() waits for the buffer, ahead() runs after the volume
+// k-steps.
+template <class C, class Flow, class Wait, class Ahead>
+__device__ __forceinline__ bool sym_adv_tile(const SymAdvOp &op, double *u, const Flow &fl,
+                                             const int4 *P, const double *ubase,
+                                             const double (&s)[4], double *kt, double dt,
+                                             double rka, double rkb, bool use_k, bool rhs_only,
+                                             int lane, Wait wait, Ahead ahead) {
   constexpr int Np = C::Np, Nfp = C::Nfp, E = C::E, MTT = C::MTT, MT0 = C::MT0, MTB = C::MTB,
                 KSF = C::KSF, KSV = C::KSV, FH = C::FH;
-  extern __shared__ __align__(16) double smem[];
-  double *sA = smem, *sBuf = sA + C::S_A;
-  unsigned long long *bars = reinterpret_cast<unsigned long long *>(sBuf + NW * 2 * C::S_U);
-  int *tabs = reinterpret_cast<int *>(bars + NW * 2);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (lane == 0) {
-    mbar_init(&bars[2 * warp], 1);
-    mbar_init(&bars[2 * warp + 1], 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  const long stride = (long)gridDim.x * NW, t0 = blockIdx.x + (long)gridDim.x * warp;
-  double *buf = sBuf + warp * 2 * C::S_U;
-  unsigned long long *full = bars + 2 * warp;
-  auto fetch = [&](long t, int b) {   // lane 0
-    mbar_arrive_expect_tx(&full[b], 8u * C::S_U);
-    bulk_g2s(buf + b * C::S_U, a.u_in + t * C::S_U, 8u * C::S_U, &full[b]);
-  };
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  if (lane == 0 && t0 < ntiles) fetch(t0, 0);
-  {
-    const double2 *src = reinterpret_cast<const double2 *>(a.AT);
-    double2 *dst = reinterpret_cast<double2 *>(sA);
-    for (int i = tid; i < C::S_A / 2; i += C::THREADS) dst[i] = __ldg(src + i);
-    const int *ts = reinterpret_cast<const int *>(a.AT + C::S_A);
-    // volume entries with the images' nodes in place of the shuffle lanes
-    for (int i = tid; i < KSV * 4; i += C::THREADS) {
-      const int q = i & ~3, x = __ldg(ts + i);
-      tabs[i] = (__ldg(ts + (q | ((x >> 16) & 3))) & 0x3ff) |
-                (__ldg(ts + (q | ((x >> 18) & 3))) & 0x3ff) << 10 |
-                (__ldg(ts + (q | ((x >> 20) & 3))) & 0x3ff) << 20;
-    }
-    for (int i = tid; i < C::T_FACE + C::T_OUT; i += C::THREADS)
-      tabs[KSV * 4 + i] = __ldg(ts + C::T_VOL + i);
-  }
-  __syncthreads();
-  const int *tvol = tabs;
-  const int4 *tface = reinterpret_cast<const int4 *>(tabs + KSV * 4);
-  const int4 *tout = tface + C::T_FACE / 4;
-  const int *ft = reinterpret_cast<const int *>(a.AT + C::S_A) + C::T_VOL + C::T_FACE + C::T_OUT;
-  const int f0 = __ldg(ft), f1 = __ldg(ft + 1), f2 = __ldg(ft + 2), f3 = __ldg(ft + 3);
-  const double dt = a.rhs_only ? 1.0 : a.dt_override >= 0 ? a.dt_override : a.sc->dt;
-  const bool use_k = !a.rhs_only && a.rka != 0.0;
-  const int l = lane & 3, row = lane >> 2, el = C::elem(lane >> 2);
+  const int l = lane & 3, row = lane >> 2;
+  const double *uE = u + C::elem(lane >> 2) * Np;
   auto mt0 = [](int c) { return c == 0 ? 0 : MT0 + (c - 1) * MTB; };
   double acc[MTT][2];
   auto mma = [&](int ks, double h0, double h1, double h2, double h3) {
-    const double *A = sA + (long)ks * MTT * 32 + lane;
+    const double *A = op.A + (long)ks * MTT * 32 + lane;
 #pragma unroll
     for (int m = 0; m < MT0; m++) dmma(acc[m], A[m * 32], h0);
 #pragma unroll
@@ -100,124 +110,160 @@ __global__ void __launch_bounds__(32 * NW, 1)
       dmma(acc[mt0(3) + m], A[(mt0(3) + m) * 32], h3);
     }
   };
+  // neighbours, then the first traces: on their way under the volume k-steps
+  int4 nb[KSF];
+#pragma unroll
+  for (int f = 0; f < KSF; f++) nb[f] = __ldg(P + f * 32);
+#pragma unroll
+  for (int m = 0; m < MTT; m++) acc[m][0] = acc[m][1] = 0.0;
+  double up[FH][4];
+  auto gather = [&](int f, double (&x)[4]) {
+    x[0] = __ldg(ubase + nb[f].x);
+    x[1] = __ldg(ubase + nb[f].y);
+    x[2] = __ldg(ubase + nb[f].z);
+    x[3] = __ldg(ubase + nb[f].w);
+  };
+#pragma unroll
+  for (int f = 0; f < FH; f++) gather(f, up[f]);
+  if (!wait()) return false;
+#pragma unroll 4
+  for (int ks = 0; ks < KSV; ks++) {
+    const int n = op.tvol[ks * 4 + l];
+    const double u1 = uE[n & 0x3ff], u2 = uE[(n >> 10) & 0x3ff], u3 = uE[n >> 20];
+    const double v1 = fl.vol(ks, 0), v2 = fl.vol(ks, 1), v3 = fl.vol(ks, 2);
+    const double p3 = u3 * v3, sum = fma(u2, v2, p3), d = fma(u2, v2, -p3);
+    mma(ks, fma(u1, v1, sum), fma(u1, v1, -sum), fma(-u1, v1, d), -fma(u1, v1, d));
+  }
+  ahead();
+  auto face = [&](int f, const double (&x)[4]) {
+    // (padding positions repeat the last point: finite values, zero columns)
+    const int4 q = op.tface[min(f * 4 + l, Nfp - 1)];
+    const double w0 = fl.face(f, 0), w1 = fl.face(f, 1), w2 = fl.face(f, 2), w3 = fl.face(f, 3);
+    const double p0 = fma(uE[q.x & 0xffff], w0 + s[0], x[0] * (w0 - s[0]));
+    const double p1 = fma(uE[q.y & 0xffff], w1 + s[1], x[1] * (w1 - s[1]));
+    const double p2 = fma(uE[q.z & 0xffff], w2 + s[2], x[2] * (w2 - s[2]));
+    const double p3 = fma(uE[q.w & 0xffff], w3 + s[3], x[3] * (w3 - s[3]));
+    const double a0 = p0 + p1, a1 = p0 - p1, c = p2 + p3, d = p2 - p3;
+    mma(KSV + f, a0 + c, a0 - c, a1 + d, a1 - d);
+  };
+  kt += 2 * l;
+#pragma unroll
+  for (int f = 0; f < FH; f++) face(f, up[f]);
+  // the other traces and the register
+#pragma unroll
+  for (int f = FH; f < KSF; f++) gather(f, up[f - FH]);
+  double2 kr[MTT];
+#pragma unroll
+  for (int c = 0; c < 4; c++)
+#pragma unroll
+    for (int m = 0; m < (c == 0 ? MT0 : MTB); m++) {
+      const int r = C::krow(c, 8 * m + row);
+      kr[mt0(c) + m] = make_double2(0.0, 0.0);
+      if (use_k && r >= 0) kr[mt0(c) + m] = *reinterpret_cast<const double2 *>(kt + r * E);
+    }
+#pragma unroll
+  for (int f = FH; f < KSF; f++) face(f, up[f - FH]);
+  // acc = dt rhs + rka k, the new register; u += rkb * y, y from the four characters
+  double un[MT0][2][4];
+  int4 nd[MT0];
+  double *const ue[2] = {u + C::elem(2 * l) * Np, u + C::elem(2 * l + 1) * Np};
+  __syncwarp();   // u has been read for the last fluxes
+#pragma unroll
+  for (int m = 0; m < MT0; m++) {
+    nd[m] = op.tout[8 * m + row];   // (empty slots name node 0)
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      un[m][h][0] = ue[h][nd[m].x], un[m][h][1] = ue[h][nd[m].y];
+      un[m][h][2] = ue[h][nd[m].z], un[m][h][3] = ue[h][nd[m].w];
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 4; c++)
+#pragma unroll
+    for (int m = 0; m < (c == 0 ? MT0 : MTB); m++) {
+      const int r = C::krow(c, 8 * m + row), i = mt0(c) + m;
+      acc[i][0] = dt * acc[i][0] + rka * kr[i].x;
+      acc[i][1] = dt * acc[i][1] + rka * kr[i].y;
+      if (!rhs_only && r >= 0)
+        *reinterpret_cast<double2 *>(kt + r * E) = make_double2(acc[i][0], acc[i][1]);
+    }
+  __syncwarp();   // every lane has its old values
+#pragma unroll
+  for (int m = 0; m < MT0; m++)
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const double y0 = acc[m][h];
+      double y1, y2, y3;
+      sym_characters<C>(acc, m, h, row, lane, y1, y2, y3);
+      const double s01 = y0 + y1, d01 = y0 - y1, s23 = y2 + y3, d23 = y2 - y3;
+      const double *const o = un[m][h];
+      if (8 * m + row < C::R0) {
+        ue[h][nd[m].x] = rhs_only ? s01 + s23 : o[0] + rkb * (s01 + s23);
+        ue[h][nd[m].y] = rhs_only ? s01 - s23 : o[1] + rkb * (s01 - s23);
+        ue[h][nd[m].z] = rhs_only ? d01 + d23 : o[2] + rkb * (d01 + d23);
+        ue[h][nd[m].w] = rhs_only ? d01 - d23 : o[3] + rkb * (d01 - d23);
+      }
+    }
+  return true;
+}
+
+template <int N, int NW>
+__global__ void __launch_bounds__(32 * NW, 1)
+    stage_sym_adv_kernel(const StageArgs a, int ntiles) {
+  using C = SymAdvCfg<N, NW>;
+  constexpr int Np = C::Np, E = C::E;
+  extern __shared__ __align__(16) double smem[];
+  double *sA = smem, *sBuf = sA + C::S_A;
+  unsigned long long *bars = reinterpret_cast<unsigned long long *>(sBuf + NW * 2 * C::S_U);
+  int *tabs = reinterpret_cast<int *>(bars + NW * 2);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  double *buf = sBuf + warp * 2 * C::S_U;
+  unsigned long long *full = bars + 2 * warp;
+  if (lane == 0) {
+    mbar_init(&full[0], 1);
+    mbar_init(&full[1], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  const long stride = (long)gridDim.x * NW, t0 = blockIdx.x + (long)gridDim.x * warp;
+  auto fetch = [&](long t, int b) {   // lane 0
+    mbar_arrive_expect_tx(&full[b], 8u * C::S_U);
+    bulk_g2s(buf + b * C::S_U, a.u_in + t * C::S_U, 8u * C::S_U, &full[b]);
+  };
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  if (lane == 0 && t0 < ntiles) fetch(t0, 0);
+  const SymAdvOp op = sym_adv_operator<C>(a.AT, sA, tabs, tid, C::THREADS);
+  __syncthreads();
+  const int *ft = reinterpret_cast<const int *>(a.AT + C::S_A) + C::T_VOL + C::T_FACE + C::T_OUT;
+  const int fo[4] = {__ldg(ft), __ldg(ft + 1), __ldg(ft + 2), __ldg(ft + 3)};
+  const double dt = a.rhs_only ? 1.0 : a.dt_override >= 0 ? a.dt_override : a.sc->dt;
+  const bool use_k = !a.rhs_only && a.rka != 0.0;
+  const int el = C::elem(lane >> 2);
   bool ok = true;
   int it = 0;
   for (long t = t0; t < ntiles; t += stride, it++) {
     const int b = it & 1;
     double *u = buf + b * C::S_U;
-    const double *uE = u + el * Np;
-    const double *V = a.erec + t * C::FLOW + lane, *W = V + C::F_V;
-    const int4 *P = reinterpret_cast<const int4 *>(a.erec + t * C::FLOW + C::F_V + C::F_W) + lane;
-    // neighbours, then the first traces: on their way under the volume k-steps
-    int4 nb[KSF];
+    const double *F = a.erec + t * C::FLOW;
+    double s[4];
 #pragma unroll
-    for (int f = 0; f < KSF; f++) nb[f] = __ldg(P + f * 32);
-    // Fscale tau / 2 of the element's faces, by label
-    double s0, s1, s2, s3;
-    {
-      const double *fs = a.fscale + (t * E + el) * 4, *ta = a.tau + (t * E + el) * 4;
-      s0 = 0.5 * __ldg(fs + f0) * __ldg(ta + f0);
-      s1 = 0.5 * __ldg(fs + f1) * __ldg(ta + f1);
-      s2 = 0.5 * __ldg(fs + f2) * __ldg(ta + f2);
-      s3 = 0.5 * __ldg(fs + f3) * __ldg(ta + f3);
-    }
-#pragma unroll
-    for (int m = 0; m < MTT; m++) acc[m][0] = acc[m][1] = 0.0;
-    double up[FH][4];
-    auto gather = [&](int f, double (&x)[4]) {
-      x[0] = __ldg(a.u_in + nb[f].x);
-      x[1] = __ldg(a.u_in + nb[f].y);
-      x[2] = __ldg(a.u_in + nb[f].z);
-      x[3] = __ldg(a.u_in + nb[f].w);
-    };
-#pragma unroll
-    for (int f = 0; f < FH; f++) gather(f, up[f]);
-    ok = __all_sync(0xffffffffu, mbar_wait(&full[b], (it >> 1) & 1, a.wait_cycles));
+    for (int v = 0; v < 4; v++)
+      s[v] = 0.5 * __ldg(a.fscale + (t * E + el) * 4 + fo[v]) *
+             __ldg(a.tau + (t * E + el) * 4 + fo[v]);
+    ok = sym_adv_tile<C>(
+        op, u, FlowRecord{F + lane, F + C::F_V + lane},
+        reinterpret_cast<const int4 *>(F + C::F_V + C::F_W) + lane, a.u_in, s,
+        a.kreg + t * C::S_U, dt, a.rka, a.rkb, use_k, a.rhs_only != 0, lane,
+        [&]() {
+          return __all_sync(0xffffffffu, mbar_wait(&full[b], (it >> 1) & 1, a.wait_cycles)) != 0;
+        },
+        [&]() {
+          // the next tile's state, once the previous tile's store has read its buffer
+          if (lane == 0 && t + stride < ntiles) {
+            bulk_wait_read();
+            fetch(t + stride, b ^ 1);
+          }
+        });
     if (!ok) break;
-#pragma unroll 4
-    for (int ks = 0; ks < KSV; ks++) {
-      const int n = tvol[ks * 4 + l];
-      const double u1 = uE[n & 0x3ff], u2 = uE[(n >> 10) & 0x3ff], u3 = uE[n >> 20];
-      const double v1 = __ldg(V + ks * 96), v2 = __ldg(V + ks * 96 + 32),
-                   v3 = __ldg(V + ks * 96 + 64);
-      const double p3 = u3 * v3, s = fma(u2, v2, p3), d = fma(u2, v2, -p3);
-      mma(ks, fma(u1, v1, s), fma(u1, v1, -s), fma(-u1, v1, d), -fma(u1, v1, d));
-    }
-    // the next tile's state, once the previous tile's store has read its buffer
-    if (lane == 0 && t + stride < ntiles) {
-      bulk_wait_read();
-      fetch(t + stride, b ^ 1);
-    }
-    double2 kr[MTT];
-    auto face = [&](int f, const double (&x)[4]) {
-      // (padding positions repeat the last point: finite values, zero columns)
-      const int4 q = tface[min(f * 4 + l, Nfp - 1)];
-      const double *w = W + f * 128;
-      const double w0 = __ldg(w), w1 = __ldg(w + 32), w2 = __ldg(w + 64), w3 = __ldg(w + 96);
-      const double p0 = fma(uE[q.x & 0xffff], w0 + s0, x[0] * (w0 - s0));
-      const double p1 = fma(uE[q.y & 0xffff], w1 + s1, x[1] * (w1 - s1));
-      const double p2 = fma(uE[q.z & 0xffff], w2 + s2, x[2] * (w2 - s2));
-      const double p3 = fma(uE[q.w & 0xffff], w3 + s3, x[3] * (w3 - s3));
-      const double a0 = p0 + p1, a1 = p0 - p1, c = p2 + p3, d = p2 - p3;
-      mma(KSV + f, a0 + c, a0 - c, a1 + d, a1 - d);
-    };
-    double *kt = a.kreg + t * C::S_U + 2 * l;
-#pragma unroll
-    for (int f = 0; f < FH; f++) face(f, up[f]);
-    // the other traces and the register
-#pragma unroll
-    for (int f = FH; f < KSF; f++) gather(f, up[f - FH]);
-#pragma unroll
-    for (int c = 0; c < 4; c++)
-#pragma unroll
-      for (int m = 0; m < (c == 0 ? MT0 : MTB); m++) {
-        const int r = C::krow(c, 8 * m + row);
-        kr[mt0(c) + m] = make_double2(0.0, 0.0);
-        if (use_k && r >= 0)
-          kr[mt0(c) + m] = *reinterpret_cast<const double2 *>(kt + r * E);
-      }
-#pragma unroll
-    for (int f = FH; f < KSF; f++) face(f, up[f - FH]);
-    // acc = dt rhs + rka k, the new register; u += rkb * y, y from the four characters
-    double un[MT0][2][4];
-    int4 nd[MT0];
-    double *const ue[2] = {u + C::elem(2 * l) * Np, u + C::elem(2 * l + 1) * Np};
-    __syncwarp();   // u has been read for the last fluxes
-#pragma unroll
-    for (int m = 0; m < MT0; m++) {
-      nd[m] = tout[8 * m + row];   // (empty slots name node 0)
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        un[m][h][0] = ue[h][nd[m].x], un[m][h][1] = ue[h][nd[m].y];
-        un[m][h][2] = ue[h][nd[m].z], un[m][h][3] = ue[h][nd[m].w];
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < 4; c++)
-#pragma unroll
-      for (int m = 0; m < (c == 0 ? MT0 : MTB); m++) {
-        const int r = C::krow(c, 8 * m + row), i = mt0(c) + m;
-        acc[i][0] = dt * acc[i][0] + a.rka * kr[i].x;
-        acc[i][1] = dt * acc[i][1] + a.rka * kr[i].y;
-        if (!a.rhs_only && r >= 0)
-          *reinterpret_cast<double2 *>(kt + r * E) = make_double2(acc[i][0], acc[i][1]);
-      }
-    __syncwarp();   // every lane has its old values
-#pragma unroll
-    for (int m = 0; m < MT0; m++)
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        double y0 = acc[m][h], y1, y2, y3;
-        sym_characters<C>(acc, m, h, row, lane, y1, y2, y3);
-        const double s01 = y0 + y1, d01 = y0 - y1, s23 = y2 + y3, d23 = y2 - y3;
-        const double *const o = un[m][h];
-        if (8 * m + row < C::R0) {
-          ue[h][nd[m].x] = a.rhs_only ? s01 + s23 : o[0] + a.rkb * (s01 + s23);
-          ue[h][nd[m].y] = a.rhs_only ? s01 - s23 : o[1] + a.rkb * (s01 - s23);
-          ue[h][nd[m].z] = a.rhs_only ? d01 + d23 : o[2] + a.rkb * (d01 + d23);
-          ue[h][nd[m].w] = a.rhs_only ? d01 - d23 : o[3] + a.rkb * (d01 - d23);
-        }
-      }
     const int ne = (int)min((long)E, (long)a.K - t * E);
     if (ne < E) {
       __syncwarp();

@@ -1,0 +1,15 @@
+// Device code of the symmetry-adapted kernels for the units that use it (the
+// single-mesh stages and the batches).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "dglm_common.cuh"
+#include "dglm_ptx.cuh"
+
+namespace dglm {
+
+#include "dglm_stage_sym.cuh"
+#include "dglm_stage_sym_adv.cuh"
+
+}  // namespace dglm
