@@ -1451,11 +1451,9 @@ dglm_status dglm_adjoint_record(dglm_handle *h, int nsteps, int checkpoint_every
   t->recorded = false;
   t->capped = false;
   cudaStream_t s = h->stream;
-  const double zero = 0.0;
-  cudaError_t e = cudaMemcpyAsync(&h->sc->dt_fixed, &zero, sizeof(double),
-                                  cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return cuda_check(e, "dglm_adjoint_record");
+  st = set_dt_fixed(h, 0.0);
+  if (st != DGLM_OK) return st;
+  cudaError_t e = cudaSuccess;
   h->launches = 0;
   const bool euler = h->d.physics == DGLM_EULER;
   const int last_s0 = (nsteps - 1) / checkpoint_every * checkpoint_every;
@@ -1748,11 +1746,9 @@ dglm_status dglm_adjoint_record_capped(dglm_handle *h, int nsteps, size_t max_by
   // advection: the penalty is fixed at set-state time
   if (e == cudaSuccess && !euler)
     e = cudaMemcpyAsync(t->tau, h->tau, sizeof(double) * 4 * h->Kp, cudaMemcpyDeviceToDevice, s);
-  const double zero = 0.0;
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(&h->sc->dt_fixed, &zero, sizeof(double), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_check(e, "dglm_adjoint_record_capped");
+  st = set_dt_fixed(h, 0.0);
+  if (st != DGLM_OK) return st;
   revolve_spine(plan, nchunk, slots - 1, t->spine);
   h->launches = 0;
   size_t q = 0;

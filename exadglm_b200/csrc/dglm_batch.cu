@@ -357,6 +357,7 @@ __device__ __forceinline__ bool batch_sym_tiles(const BatchSymArgs &a, int lo, i
   const SymAdvOp op = sym_adv_operator<C>(a.image[N], smem, tabs, tid, 32 * kSymWarps);
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncthreads();
+  pdl_wait();
   bool ok = true;
   if (warp < NW && lo + warp < hi) {
     double *buf = sBuf + warp * 2 * C::S_U;
@@ -420,6 +421,7 @@ __device__ __forceinline__ bool batch_sym_tiles(const BatchSymArgs &a, int lo, i
 
 __global__ void __launch_bounds__(32 * kSymWarps, 1) batch_sym_kernel(const BatchSymArgs a) {
   extern __shared__ __align__(16) double smem[];
+  pdl_launch();
   // the warps' barriers sit behind the largest order's layout
   unsigned long long *full = reinterpret_cast<unsigned long long *>(
       reinterpret_cast<char *>(smem) + kBatchSymSmem - 16 * kSymWarps) + 2 * (threadIdx.x >> 5);
@@ -429,6 +431,7 @@ __global__ void __launch_bounds__(32 * kSymWarps, 1) batch_sym_kernel(const Batc
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   const int first = a.cut[blockIdx.x], last = a.cut[blockIdx.x + 1];
+  if (first == last) pdl_wait();   // no tile: still after the launch before
   int it = 0;
   bool ok = true;
   auto stretch = [&](int N, int &lo, int &hi) {
@@ -521,6 +524,8 @@ __global__ void batch_wavespeed_kernel(const BatchInst *inst, const double *fsca
 // advec_time.cpp), clipped so the instance ends at tmax; 0 once it has.
 __global__ void batch_step_begin_kernel(int n, const BatchInst *inst, double cfl, double tmax,
                                         BatchScalars *sc) {
+  pdl_launch();
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double m = __longlong_as_double((long long)sc[i].acc);
@@ -534,6 +539,8 @@ __global__ void batch_step_begin_kernel(int n, const BatchInst *inst, double cfl
 }
 
 __global__ void batch_step_end_kernel(int n, BatchScalars *sc) {
+  pdl_launch();
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n || !sc[i].active) return;
   sc[i].t += sc[i].dt;
@@ -661,8 +668,8 @@ void drop_batch_graphs(dglm_batch *b) {
 cudaError_t issue_batch_step(dglm_batch *b, int cur, cudaStream_t s) {
   const int n = (int)b->hinst.size();
   const int tb = 128, nb = (n + tb - 1) / tb;
-  batch_step_begin_kernel<<<nb, tb, 0, s>>>(n, b->inst, b->d.cfl, b->d.tmax, b->sc);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_pdl(batch_step_begin_kernel, dim3(nb), dim3(tb), 0, s, n, b->inst,
+                             b->d.cfl, b->d.tmax, b->sc);
   for (int st = 0; st < 5 && e == cudaSuccess; st++) {
     const int in = (cur + st) & 1;
     if (b->sym) {
@@ -671,8 +678,7 @@ cudaError_t issue_batch_step(dglm_batch *b, int cur, cudaStream_t s) {
       q.u_out = b->u[in ^ 1];
       q.rka = RKA[st];
       q.rkb = RKB[st];
-      batch_sym_kernel<<<b->grid, 32 * kSymWarps, kBatchSymSmem, s>>>(q);
-      e = cudaGetLastError();
+      e = launch_pdl(batch_sym_kernel, dim3(b->grid), dim3(32 * kSymWarps), kBatchSymSmem, s, q);
       continue;
     }
     BatchArgs a = b->args;
@@ -684,8 +690,7 @@ cudaError_t issue_batch_step(dglm_batch *b, int cur, cudaStream_t s) {
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) {
-    batch_step_end_kernel<<<nb, tb, 0, s>>>(n, b->sc);
-    e = cudaGetLastError();
+    e = launch_pdl(batch_step_end_kernel, dim3(nb), dim3(tb), 0, s, n, b->sc);
   }
   return e;
 }

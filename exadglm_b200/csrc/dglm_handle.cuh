@@ -45,6 +45,7 @@ struct dglm_handle {
   double *kreg = nullptr;
   int cur = 0;
   dglm::DevScalars *sc = nullptr;
+  double dt_fixed = -1.0;         // sc->dt_fixed as last written (-1: not known)
   double *dt_hist = nullptr;
   // one-off right-hand side evaluation
   double *rhs_in = nullptr, *rhs_out = nullptr, *maxv_s = nullptr, *tau_s = nullptr;
@@ -108,6 +109,7 @@ inline dglm_status dalloc(dglm_handle *h, T **p, size_t count) {
 StageArgs stage_args(dglm_handle *h, const double *u_in, double *u_out, int s);
 void free_tape(dglm_handle *h);
 dglm_status run_steps(dglm_handle *h, int nsteps);
+dglm_status set_dt_fixed(dglm_handle *h, double dt);
 dglm_status issue_step_ptrs(dglm_handle *h, const double *const *in, double *const *out,
                             cudaStream_t s);
 dglm_status ensure_rhs_scratch(dglm_handle *h);

@@ -8,6 +8,33 @@
 
 namespace dglm {
 
+// Programmatic dependent launch.  The kernels of a step are launched with
+// launch_pdl, so that one's start (barriers, the operator's copy to shared
+// memory) overlaps the end of the one before: each lets its successor start as
+// soon as all its blocks run, and reads nothing that an earlier kernel writes,
+// nor writes anything, before pdl_wait.
+__device__ __forceinline__ void pdl_launch() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                              cudaStream_t s, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &attr;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 __device__ __forceinline__ unsigned smem_u32(const void *p) {
   return (unsigned)__cvta_generic_to_shared(p);
 }

@@ -721,6 +721,7 @@ dglm_status dglm_set_state(dglm_handle *h, const double *const *u, int on_device
                         on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(h->kreg, 0, sizeof(double) * h->nvar * h->vs, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(h->sc, 0, sizeof(DevScalars), s);
+  h->dt_fixed = 0.0;
   if (e == cudaSuccess) e = cudaMemsetAsync(h->dt_hist, 0, sizeof(double) * kHistory, s);
   if (e != cudaSuccess) return cuda_check(e, "dglm_set_state");
   e = launch_finite_check(h->u[0], h->vs, n, h->nvar, h->sc, s);
@@ -763,6 +764,7 @@ static cudaError_t reset_for_state(dglm_handle *h, cudaStream_t s) {
   h->cur = 0;
   cudaError_t e = cudaMemsetAsync(h->kreg, 0, sizeof(double) * h->nvar * h->vs, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(h->sc, 0, sizeof(DevScalars), s);
+  h->dt_fixed = 0.0;
   if (e == cudaSuccess) e = cudaMemsetAsync(h->dt_hist, 0, sizeof(double) * kHistory, s);
   if (e == cudaSuccess)
     e = launch_finite_check(h->u[0], h->vs, (long)h->d.K * h->Np, h->nvar, h->sc, s);
@@ -924,18 +926,26 @@ dglm_status dglm::run_steps(dglm_handle *h, int nsteps) {
   return DGLM_OK;
 }
 
+// Prescribed dt of the coming steps on the device (0: the CFL dt).  Written only
+// when it changes: the copy from pageable memory waits for the stream.
+dglm_status dglm::set_dt_fixed(dglm_handle *h, double dt) {
+  if (h->dt_fixed == dt) return DGLM_OK;
+  cudaError_t e = cudaMemcpyAsync(&h->sc->dt_fixed, &dt, sizeof(double), cudaMemcpyHostToDevice,
+                                  h->stream);
+  // the pageable source must stay alive until the copy is staged
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+  if (e != cudaSuccess) return cuda_check(e, "dglm_step");
+  h->dt_fixed = dt;
+  return DGLM_OK;
+}
+
 extern "C" {
 
 dglm_status dglm_step(dglm_handle *h, int nsteps) {
   if (!h) return set_error(DGLM_ERR_INVALID, "dglm_step: NULL handle");
   DeviceGuard g(h->dev);
-  const double zero = 0.0;
-  cudaError_t e = cudaMemcpyAsync(&h->sc->dt_fixed, &zero, sizeof(double),
-                                  cudaMemcpyHostToDevice, h->stream);
-  if (e != cudaSuccess) return cuda_check(e, "dglm_step");
-  // the pageable source must stay alive until the copy is staged
-  e = cudaStreamSynchronize(h->stream);
-  if (e != cudaSuccess) return cuda_check(e, "dglm_step");
+  dglm_status st = set_dt_fixed(h, 0.0);
+  if (st != DGLM_OK) return st;
   h->launches = 0;
   return run_steps(h, nsteps);
 }
@@ -945,10 +955,8 @@ dglm_status dglm_step_fixed_dt(dglm_handle *h, int nsteps, double dt) {
   if (!(dt > 0) || !std::isfinite(dt))
     return set_error(DGLM_ERR_INVALID, "dglm_step_fixed_dt: dt must be positive and finite");
   DeviceGuard g(h->dev);
-  cudaError_t e = cudaMemcpyAsync(&h->sc->dt_fixed, &dt, sizeof(double),
-                                  cudaMemcpyHostToDevice, h->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  if (e != cudaSuccess) return cuda_check(e, "dglm_step_fixed_dt");
+  dglm_status st = set_dt_fixed(h, dt);
+  if (st != DGLM_OK) return st;
   h->launches = 0;
   return run_steps(h, nsteps);
 }

@@ -670,7 +670,9 @@ __global__ void __launch_bounds__(256, kMaxvBlocksPerSM)
   __shared__ int sFm[NFF];
   __shared__ unsigned long long sMax[8];
   const int t = threadIdx.x;
+  pdl_launch();
   for (int i = t; i < NFF; i += blockDim.x) sFm[i] = a.Fmask[i];
+  pdl_wait();
   const double *src = PHYS == EUL ? a.u_in : a.vel;
   double q[NQ];
   auto fetch = [&](long e0) {
@@ -733,6 +735,8 @@ __global__ void __launch_bounds__(256, kMaxvBlocksPerSM)
 // of the new state into the other slot.
 __global__ void step_begin_kernel(int N, double cfl, double tmax, int frozen, DevScalars *sc,
                                   double *dt_hist) {
+  pdl_launch();
+  pdl_wait();
   if (threadIdx.x != 0) return;
   const int p = frozen ? 0 : sc->parity;
   const double m = __longlong_as_double((long long)sc->acc[p]);
@@ -759,6 +763,8 @@ __global__ void finite_check_kernel(const double *__restrict__ u, long vs, long 
 }
 
 __global__ void step_end_kernel(DevScalars *sc) {
+  pdl_launch();
+  pdl_wait();
   if (threadIdx.x != 0) return;
   if (sc->active) {
     sc->t += sc->dt;
@@ -770,6 +776,8 @@ __global__ void step_end_kernel(DevScalars *sc) {
 // update_tau (euler_dglm.cpp:72-84)
 __global__ void tau_kernel(int K, double tau_scale, const int *__restrict__ vmapF,
                            const double *__restrict__ maxv, double *__restrict__ tau) {
+  pdl_launch();
+  pdl_wait();
   const long f = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (f < 4L * K) tau[f] = 0.25 * (maxv[f] + maxv[vmapF[f]]) * tau_scale;
 }
@@ -1128,8 +1136,7 @@ static cudaError_t launch_maxv_one(const StageArgs &a, int slot, cudaStream_t s)
   constexpr int ET = 256 / np_of(N);
   long blocks = (a.K + ET - 1) / ET;
   if (blocks > (long)kMaxvBlocksPerSM * sm_count()) blocks = (long)kMaxvBlocksPerSM * sm_count();
-  face_maxv_kernel<PHYS, N><<<(int)blocks, 256, 0, s>>>(a, slot);
-  return cudaGetLastError();
+  return launch_pdl(face_maxv_kernel<PHYS, N>, dim3((unsigned)blocks), dim3(256), 0, s, a, slot);
 }
 
 cudaError_t launch_face_maxv(int physics, int N, const StageArgs &a, int slot,
@@ -1149,15 +1156,14 @@ cudaError_t launch_face_maxv(int physics, int N, const StageArgs &a, int slot,
 
 cudaError_t launch_step_begin(int N, double cfl, double tmax, int frozen, DevScalars *sc,
                               double *dt_hist, cudaStream_t s) {
-  step_begin_kernel<<<1, 32, 0, s>>>(N, cfl, tmax, frozen, sc, dt_hist);
-  return cudaGetLastError();
+  return launch_pdl(step_begin_kernel, dim3(1), dim3(32), 0, s, N, cfl, tmax, frozen, sc, dt_hist);
 }
 
 cudaError_t launch_tau(int K, double tau_scale, const int *vmapF, const double *maxv,
                        double *tau, cudaStream_t s) {
   const long n = 4L * K;
-  tau_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(K, tau_scale, vmapF, maxv, tau);
-  return cudaGetLastError();
+  return launch_pdl(tau_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, s, K, tau_scale,
+                    vmapF, maxv, tau);
 }
 
 cudaError_t launch_finite_check(const double *u, long vs, long n, int nvar, DevScalars *sc,
@@ -1167,8 +1173,7 @@ cudaError_t launch_finite_check(const double *u, long vs, long n, int nvar, DevS
 }
 
 cudaError_t launch_step_end(DevScalars *sc, cudaStream_t s) {
-  step_end_kernel<<<1, 32, 0, s>>>(sc);
-  return cudaGetLastError();
+  return launch_pdl(step_end_kernel, dim3(1), dim3(32), 0, s, sc);
 }
 
 }  // namespace dglm

@@ -303,8 +303,7 @@ cudaError_t launch_sym(const StageArgs &a, cudaStream_t s) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (sms <= 0) sms = 148;
   const int ntiles = (a.K + C::E - 1) / C::E;
-  k<<<ntiles < sms ? ntiles : sms, C::THREADS, C::SMEM, s>>>(a, ntiles);
-  return cudaGetLastError();
+  return launch_pdl(k, dim3(ntiles < sms ? ntiles : sms), dim3(C::THREADS), C::SMEM, s, a, ntiles);
 }
 
 template <int N, int NS, int NG, int NB>
@@ -336,8 +335,7 @@ cudaError_t launch_sym_adv(const StageArgs &a, cudaStream_t s) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (sms <= 0) sms = 148;
   const int ntiles = (a.K + C::E - 1) / C::E;
-  k<<<ntiles < sms ? ntiles : sms, C::THREADS, C::SMEM, s>>>(a, ntiles);
-  return cudaGetLastError();
+  return launch_pdl(k, dim3(ntiles < sms ? ntiles : sms), dim3(C::THREADS), C::SMEM, s, a, ntiles);
 }
 
 template <int N, int NW>

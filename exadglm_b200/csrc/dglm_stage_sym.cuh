@@ -705,6 +705,7 @@ __global__ void __launch_bounds__(SymCfg<N, NS, NG, NB>::THREADS, 1)
   r.seq = reinterpret_cast<volatile int *>(r.dump + NG);
   int *tabs = reinterpret_cast<int *>(r.full + C::NBAR);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  pdl_launch();
   if (tid == 0) {
     for (int i = 0; i < NB; i++) {
       mbar_init(&r.full[i], 1);
@@ -728,6 +729,7 @@ __global__ void __launch_bounds__(SymCfg<N, NS, NG, NB>::THREADS, 1)
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncthreads();
+  pdl_wait();
   if (warp >= C::NWC) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::REGP));
     const int lw = warp - C::NWC;

@@ -229,10 +229,12 @@ __global__ void __launch_bounds__(32 * NW, 1)
     mbar_arrive_expect_tx(&full[b], 8u * C::S_U);
     bulk_g2s(buf + b * C::S_U, a.u_in + t * C::S_U, 8u * C::S_U, &full[b]);
   };
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  if (lane == 0 && t0 < ntiles) fetch(t0, 0);
+  pdl_launch();
   const SymAdvOp op = sym_adv_operator<C>(a.AT, sA, tabs, tid, C::THREADS);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncthreads();
+  pdl_wait();
+  if (lane == 0 && t0 < ntiles) fetch(t0, 0);
   const int *ft = reinterpret_cast<const int *>(a.AT + C::S_A) + C::T_VOL + C::T_FACE + C::T_OUT;
   const int fo[4] = {__ldg(ft), __ldg(ft + 1), __ldg(ft + 2), __ldg(ft + 3)};
   const double dt = a.rhs_only ? 1.0 : a.dt_override >= 0 ? a.dt_override : a.sc->dt;
