@@ -894,8 +894,7 @@ static cudaError_t launch_tc(const StageArgs &a, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   const int ntiles = (a.K + E - 1) / E;
   const int grid = ntiles < sm_count() ? ntiles : sm_count();
-  k<<<grid, C::THREADS, C::SMEM, s>>>(a, ntiles);
-  return cudaGetLastError();
+  return launch_pdl(k, dim3(grid), dim3(C::THREADS), C::SMEM, s, a, ntiles);
 }
 
 template <int PHYS, int N, int E, int NF, int NB, bool DB, bool DF>
@@ -907,8 +906,7 @@ static cudaError_t launch_tcb(const StageArgs &a, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   const int ntiles = (a.K + E - 1) / E;
   const int grid = ntiles < sm_count() ? ntiles : sm_count();
-  k<<<grid, C::THREADS, C::SMEM, s>>>(a, ntiles);
-  return cudaGetLastError();
+  return launch_pdl(k, dim3(grid), dim3(C::THREADS), C::SMEM, s, a, ntiles);
 }
 
 template <int PHYS, int N, int E, int NF, int NB, bool DB, bool DF = false>

@@ -166,6 +166,28 @@ __device__ __forceinline__ void tmem_st8(unsigned taddr, const unsigned (&r)[8])
 __device__ __forceinline__ void tmem_st_wait() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
+// KT columns of a lane's row of the operator image (img, 16-byte aligned) into
+// tensor memory from column address col, 32 columns of 16-byte loads in flight
+// at a time.  (Eight 4-byte loads at a time left the start of every stage
+// waiting for some 20 (TF32, N=4) to 46 (BF16, N=6) round trips to L2.)
+template <int KT>
+__device__ __forceinline__ void operator_to_tmem(const unsigned *img, unsigned col) {
+  static_assert(KT % 8 == 0, "whole 8-column stores");
+#pragma unroll 1
+  for (int c = 0; c < KT; c += 32) {
+    uint4 q[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+      if (c + 4 * i < KT) q[i] = __ldg(reinterpret_cast<const uint4 *>(img + c) + i);
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (c + 8 * j < KT) {
+        unsigned r[8] = {q[2 * j].x,     q[2 * j].y,     q[2 * j].z,     q[2 * j].w,
+                         q[2 * j + 1].x, q[2 * j + 1].y, q[2 * j + 1].z, q[2 * j + 1].w};
+        tmem_st8(col + c + 8 * j, r);
+      }
+  }
+}
 __device__ __forceinline__ void tmem_ld4(unsigned taddr, float *r) {
   unsigned v[4];
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
@@ -209,6 +231,7 @@ __global__ void __launch_bounds__(TCfg<PHYS, N, E_, NC_, NB_, NPL_, DF_>::THREAD
   auto ring = [&](int it) { return sRing + (it % NB) * C::S_BUF; };
   auto tile_e0 = [&](int it) { return ((long)blockIdx.x + (long)it * gridDim.x) * E; };
 
+  pdl_launch();
   if (tid == 0) {
     for (int b = 0; b < NB; b++) {
       mbar_init(&full[b], 1 + 32);   // the byte-count arrive + each producer lane's gathers
@@ -238,18 +261,13 @@ __global__ void __launch_bounds__(TCfg<PHYS, N, E_, NC_, NB_, NPL_, DF_>::THREAD
   if (warp < 4) {
     const unsigned *img =
         reinterpret_cast<const unsigned *>(a.AT) + (size_t)(32 * warp + lane) * C::KT;
-#pragma unroll 1
-    for (int c = 0; c < C::KT; c += 8) {
-      unsigned r[8];
-#pragma unroll
-      for (int i = 0; i < 8; i++) r[i] = __ldg(img + c + i);
-      tmem_st8(tmem + ((unsigned)(32 * warp) << 16) + C::A_COL + c, r);
-    }
+    operator_to_tmem<C::KT>(img, tmem + ((unsigned)(32 * warp) << 16) + C::A_COL);
     tmem_st_wait();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
 
   const double dt = a.dt_override >= 0 ? a.dt_override : a.sc->dt;
   const double gam = a.gamma;

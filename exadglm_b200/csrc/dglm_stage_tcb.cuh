@@ -143,6 +143,7 @@ __global__ void __launch_bounds__(TBCfg<PHYS, N, E_, NC_, NB_, DBUF_, DF_>::THRE
   auto bsel = [&](int t) { return DBUF_ ? (t & 1) : 0; };
   auto bphase = [&](int t) { return DBUF_ ? ((t >> 1) & 1) : (t & 1); };
 
+  pdl_launch();
   if (tid == 0) {
     for (int b = 0; b < NB; b++) {
       mbar_init(&full[b], 1 + 32);
@@ -170,18 +171,13 @@ __global__ void __launch_bounds__(TBCfg<PHYS, N, E_, NC_, NB_, DBUF_, DF_>::THRE
   if (warp < 4) {
     const unsigned *img =
         reinterpret_cast<const unsigned *>(a.AT) + (size_t)(32 * warp + lane) * C::KT;
-#pragma unroll 1
-    for (int c = 0; c < C::KT; c += 8) {
-      unsigned r[8];
-#pragma unroll
-      for (int i = 0; i < 8; i++) r[i] = __ldg(img + c + i);
-      tmem_st8(tmem + ((unsigned)(32 * warp) << 16) + C::A_COL + c, r);
-    }
+    operator_to_tmem<C::KT>(img, tmem + ((unsigned)(32 * warp) << 16) + C::A_COL);
     tmem_st_wait();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
 
   const double dt = a.dt_override >= 0 ? a.dt_override : a.sc->dt;
   const double gam = a.gamma;
