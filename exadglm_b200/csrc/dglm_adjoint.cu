@@ -478,12 +478,20 @@ struct DCfg {
 // takes m-tiles w, w + WARPS, ... of the MTX m-tiles (A fragments [kstep]
 // [mtile][lane] from global memory, one load per k-step for NT DMMAs), the B
 // fragments come from the mu rows in shared memory; results for rows below
-// `rows` go to sOut[(v E + e) RLD + row].
+// `rows` go to sOut[(v E + e) RLD + row].  The fragments come from L2 (three
+// CTAs leave L1 too small for them), so up to 9 k-steps' loads are in flight
+// (N=4: the whole m-tile's).  With that, a tile's fields loaded before any is
+// stored, and the node's face points found by all threads at once, a backward
+// step (Euler N=4, K=24,576) went from 1.022 to 0.878 ms, K=82,944 3.145 to
+// 2.757.  Measured and not kept: programmatic dependent launch of this kernel
+// and the face kernel (1.023, 3.314: the waiting blocks hold the shared memory
+// that the running kernel's next blocks need).
 template <class C>
 __device__ __forceinline__ void adj_contract_all_n(const double *A, int MTX, int rows,
                                                    const double *sB, double *sOut, int warp,
                                                    int lane) {
   constexpr int NT = C::NT, E = C::E;
+  constexpr int PF = C::KS < 9 ? C::KS : 9;   // operator fragments in flight
   // rows k0 + (lane & 3), k0 % 4 == 0: the swizzle bit is lane bit 1
   const double *Bb = sB + (lane & 3) * C::BLD + C::bcol(lane & 3, lane >> 2);
   for (int mt = warp; mt < MTX; mt += C::WARPS) {
@@ -491,11 +499,13 @@ __device__ __forceinline__ void adj_contract_all_n(const double *A, int MTX, int
 #pragma unroll
     for (int j = 0; j < NT; j++) acc[j][0] = acc[j][1] = 0.0;
     const double *Ab = A + (long)mt * 32 + lane;
-    double an = __ldg(Ab);
-#pragma unroll 3
+    double an[PF];
+#pragma unroll
+    for (int ks = 0; ks < PF; ks++) an[ks] = __ldg(Ab + (long)ks * MTX * 32);
+#pragma unroll
     for (int ks = 0; ks < C::KS; ks++) {
-      const double av = an;
-      if (ks + 1 < C::KS) an = __ldg(Ab + (long)(ks + 1) * MTX * 32);
+      const double av = an[ks % PF];
+      if (ks + PF < C::KS) an[ks % PF] = __ldg(Ab + (long)(ks + PF) * MTX * 32);
 #pragma unroll
       for (int j = 0; j < NT; j++) adj_dmma(acc[j], av, Bb[ks * 4 * C::BLD + j * 8]);
     }
@@ -540,22 +550,31 @@ __global__ void __launch_bounds__(DCfg<PHYS, N, E_, MG_, SPLIT>::T, MINB)
 
   // ---- staging ------------------------------------------------------------
   for (int i = tid; i < NFF; i += T) sFm[i] = __ldg(a.Fmask + i);
-  for (int i = tid; i < Np; i += T) {
-    int c = 0;
-    for (int fj = 0; fj < NFF; fj++)
-      if (__ldg(a.Fmask + fj) == i && c < 4) sNF[i * 4 + c++] = fj;
-    for (; c < 4; c++) sNF[i * 4 + c] = -1;
-  }
+  for (int i = tid; i < 4 * Np; i += T) sNF[i] = -1;
+  if (upd)
+    for (int g = tid; g < 9 * E; g += T) {
+      const int m = g / E, e = g - m * E;
+      sGeo[g] = e < ne ? __ldg(a.geo + (long)m * a.gstride + e0 + e) : 0.0;
+    }
   const double bm = upd ? a.rkb : a.rkb_next;
-  for (int v = 0; v < NV; v++) {
-    const long base = v * vs + e0 * Np;
-    for (int g = tid; g < E * Np; g += T) {
-      const int e = g / Np, i = g - e * Np;
-      const bool ok = g < ne * Np;
+  // all variables' loads before the first store: their latencies overlap
+  for (int g = tid; g < E * Np; g += T) {
+    const int e = g / Np, i = g - e * Np;
+    const bool ok = g < ne * Np;
+    const long base = e0 * Np + g;
+    double l[NV], k[NV], q[NV];
+#pragma unroll
+    for (int v = 0; v < NV; v++) {
+      l[v] = ok ? a.lam[v * vs + base] : 0.0;
+      k[v] = ok ? a.lk[v * vs + base] : 0.0;
+      q[v] = upd && ok ? __ldg(a.u + v * vs + base) : (v == 0 ? 1.0 : 0.0);
+    }
+#pragma unroll
+    for (int v = 0; v < NV; v++) {
       const int s = (v * E + e) * C::IP + i;
-      sLam[s] = ok ? a.lam[base + g] : 0.0;
-      sOut[s] = ok ? a.lk[base + g] : 0.0;   // lk, until mu is formed below
-      if (upd) sU[s] = ok ? __ldg(a.u + base + g) : (v == 0 ? 1.0 : 0.0);
+      sLam[s] = l[v];
+      sOut[s] = k[v];   // lk, until mu is formed below
+      if (upd) sU[s] = q[v];
     }
   }
   for (int g = tid; g < (KP - Np) * BLD; g += T) sB[Np * BLD + g] = 0.0;
@@ -566,11 +585,16 @@ __global__ void __launch_bounds__(DCfg<PHYS, N, E_, MG_, SPLIT>::T, MINB)
     const int s = (v * E + e) * C::IP + i;
     sB[i * BLD + C::bcol(i, v * E + e)] = sOut[s] + bm * sLam[s];
   }
+  // face points of a node, in ascending order: a point's place is the number of
+  // earlier points on its node
+  for (int fj = tid; fj < NFF; fj += T) {
+    const int node = sFm[fj];
+    int c = 0;
+#pragma unroll 4
+    for (int q = 0; q < NFF; q++) c += q < fj && sFm[q] == node;
+    if (c < 4) sNF[node * 4 + c] = fj;
+  }
   if (upd) {
-    for (int g = tid; g < 9 * E; g += T) {
-      const int m = g / E, e = g - m * E;
-      sGeo[g] = e < ne ? __ldg(a.geo + (long)m * a.gstride + e0 + e) : 0.0;
-    }
     for (int g = tid; g < (SPLIT ? 0 : 4 * E); g += T) {
       const int e = g >> 2, f = g & 3;
       const bool ok = e < ne;
