@@ -36,7 +36,8 @@ def nvcc():
 
 
 def _deps():
-    hdrs = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(INCLUDE, "*.h"))
+    hdrs = [h for pat in (os.path.join(CSRC, "*.cuh"), os.path.join(CSRC, "*.h"),
+                          os.path.join(INCLUDE, "*.h")) for h in glob.glob(pat)]
     return max((os.path.getmtime(h) for h in hdrs), default=0.0)
 
 

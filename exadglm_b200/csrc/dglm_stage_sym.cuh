@@ -521,8 +521,8 @@ __device__ __forceinline__ void sym_mover(const StageArgs &a, int ntiles, const 
   if (!ok) {
     // an expired wait: the copies of the tiles in flight settle before the warp leaves
     if (lane == 0) atomicOr(&a.sc->flags, 4);
-    for (int q = it - C::NM; q >= 0 && q > it - NB; q -= C::NM)
-      if (q < total) mbar_wait(&r.full[q % NB], (q / NB) & 1);
+    mover_in_flight<NB, C::NM>(it, total,
+                               [&](int q) { mbar_wait(&r.full[q % NB], (q / NB) & 1); });
   }
   if (copies) bulk_wait_all();
 }

@@ -6,6 +6,7 @@
 
 #include "dglm_common.cuh"
 #include "dglm_ptx.cuh"
+#include "dglm_ring.h"
 
 namespace dglm {
 
