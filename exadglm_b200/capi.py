@@ -35,8 +35,8 @@ EXPORTS = (
     "dglm_calc_maxv_dt_static", "dglm_adjoint_variant_count", "dglm_adjoint_variant_describe",
     "dglm_adjoint_set_variant", "dglm_batch_create", "dglm_batch_add", "dglm_batch_finalize",
     "dglm_batch_step", "dglm_batch_sync", "dglm_batch_count", "dglm_batch_get_state",
-    "dglm_batch_get_time", "dglm_batch_set_stream", "dglm_batch_kernel_launches",
-    "dglm_batch_device_bytes", "dglm_batch_destroy",
+    "dglm_batch_get_time", "dglm_batch_set_stream", "dglm_batch_set_wait_limit",
+    "dglm_batch_kernel_launches", "dglm_batch_device_bytes", "dglm_batch_destroy",
 )
 
 
@@ -140,6 +140,7 @@ def lib():
         L.dglm_batch_get_state.argtypes = [_P, I, _P, I]
         L.dglm_batch_get_time.argtypes = [_P, I, C.POINTER(D), C.POINTER(D), C.POINTER(I)]
         L.dglm_batch_set_stream.argtypes = [_P, _P]
+        L.dglm_batch_set_wait_limit.argtypes = [_P, C.c_longlong]
         L.dglm_batch_kernel_launches.argtypes = [_P]
         L.dglm_batch_kernel_launches.restype = C.c_long
         L.dglm_batch_device_bytes.argtypes = [_P]
@@ -554,6 +555,11 @@ class BatchSolver:
 
     def set_stream(self, stream_ptr):
         check(self.L.dglm_batch_set_stream(self.h, C.c_void_p(int(stream_ptr))))
+
+    def set_wait_limit(self, cycles):
+        """Bound (SM clock cycles) of the stage kernel's waits; 0 restores the
+        default."""
+        check(self.L.dglm_batch_set_wait_limit(self.h, int(cycles)))
 
     def kernel_launches(self):
         return int(self.L.dglm_batch_kernel_launches(self.h))

@@ -323,6 +323,7 @@ struct BatchSymArgs {
   double *u_out, *kreg;
   double rka, rkb;
   int *err;                   // set when a bounded wait expired
+  long long wait_cycles;      // bound of the waits for a tile's state
 };
 
 // Per element: (grad r_a + sum_b grad r_b) . v (a = 1..3), Fscale n . v / 2 and
@@ -394,7 +395,9 @@ __device__ __forceinline__ bool batch_sym_tiles(const BatchSymArgs &a, int lo, i
           reinterpret_cast<const int4 *>(a.nb[N]) + (long)(ti - a.begin[N]) * P4 + lane,
           a.u_in + I.node_off, s, a.kreg + node0, a.sc[t.inst].dt, a.rka, a.rkb, a.rka != 0.0,
           false, lane,
-          [&]() { return __all_sync(0xffffffffu, mbar_wait(&full[b], (it >> 1) & 1)) != 0; },
+          [&]() {
+            return __all_sync(0xffffffffu, mbar_wait(&full[b], (it >> 1) & 1, a.wait_cycles)) != 0;
+          },
           [&]() {
             // the next tile's state, once the previous tile's store has read its buffer
             if (lane == 0 && ti + NW < hi) {
@@ -404,6 +407,7 @@ __device__ __forceinline__ bool batch_sym_tiles(const BatchSymArgs &a, int lo, i
           });
       if (!ok) {
         if (lane == 0) *a.err = 1;
+        mbar_wait(&full[b], (it >> 1) & 1);   // the tile in flight settles
         break;
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -584,6 +588,7 @@ struct dglm_batch {
   bool sym = false;                 // all orders on the symmetry-adapted path
   BatchSymArgs sargs{};
   int *err = nullptr;
+  long long wait_cycles = kWaitCycles;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   long launches = 0;
 };
@@ -678,6 +683,7 @@ cudaError_t issue_batch_step(dglm_batch *b, int cur, cudaStream_t s) {
       q.u_out = b->u[in ^ 1];
       q.rka = RKA[st];
       q.rkb = RKB[st];
+      q.wait_cycles = b->wait_cycles;
       e = launch_pdl(batch_sym_kernel, dim3(b->grid), dim3(32 * kSymWarps), kBatchSymSmem, s, q);
       continue;
     }
@@ -1132,6 +1138,17 @@ dglm_status dglm_batch_set_stream(dglm_batch *b, void *stream) {
   if (b->own_stream) cudaStreamDestroy(b->stream);
   b->own_stream = false;
   b->stream = (cudaStream_t)stream;
+  return DGLM_OK;
+}
+
+dglm_status dglm_batch_set_wait_limit(dglm_batch *b, long long cycles) {
+  if (!b) return set_error(DGLM_ERR_INVALID, "dglm_batch_set_wait_limit: NULL batch");
+  if (cycles < 0)
+    return set_error(DGLM_ERR_INVALID, "dglm_batch_set_wait_limit: negative bound");
+  DeviceGuard g(b->dev);
+  cudaStreamSynchronize(b->stream);
+  drop_batch_graphs(b);   // the captured steps carry the bound in their arguments
+  b->wait_cycles = cycles ? cycles : kWaitCycles;
   return DGLM_OK;
 }
 

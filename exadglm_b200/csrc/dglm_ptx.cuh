@@ -76,10 +76,12 @@ __device__ __forceinline__ bool mbar_test_wait(unsigned long long *b, unsigned p
 // the default bound the thread suspends in try_wait between checks; a
 // shortened bound (dglm_set_wait_limit) polls with the non-blocking
 // test_wait, so that the bound and not try_wait's own suspension time decides
-// when the wait gives up
+// when the wait gives up; a bound of one cycle gives up without a look, so that
+// waits that rarely have to wait can be made to run out too
 __device__ __forceinline__ bool mbar_wait(unsigned long long *b, unsigned parity,
                                           long long limit = kWaitCycles) {
   if (limit < kWaitCycles) {
+    if (limit <= 1) return false;
     const long long t0 = clock64();
     while (!mbar_test_wait(b, parity))
       if (clock64() - t0 > limit) return false;

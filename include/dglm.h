@@ -183,9 +183,9 @@ int dglm_get_variant(dglm_handle *h);
  * When a wait runs out, the CTA sets an error flag, waits (with the default
  * bound) for its own copies and MMAs in flight and leaves; dglm_sync and
  * dglm_rhs then return DGLM_ERR_CUDA and the handle's state is invalid until
- * the next dglm_set_state.  A short bound makes waits expire on purpose:
- * this is how the expiry path is tested.  No counterpart in the reference,
- * whose kernels have no waits between warps. */
+ * the next dglm_set_state.  A short bound makes waits expire on purpose (a
+ * bound of 1 all of them): this is how the expiry path is tested.  No
+ * counterpart in the reference, whose kernels have no waits between warps. */
 dglm_status dglm_set_wait_limit(dglm_handle *h, long long cycles);
 /* Compact face maps.  on = 1 builds, from the uploaded vmapP (once per mesh),
  * per face (e, f) the neighbour element and a one-byte code of the
@@ -375,6 +375,12 @@ int dglm_batch_count(dglm_batch *b);
 dglm_status dglm_batch_get_state(dglm_batch *b, int index, double *u, int on_device);
 dglm_status dglm_batch_get_time(dglm_batch *b, int index, double *t, double *dt, int *tstep);
 dglm_status dglm_batch_set_stream(dglm_batch *b, void *stream);
+/* Bound of the stage kernel's waits, as dglm_set_wait_limit for a handle.
+ * After a wait ran out dglm_batch_sync returns DGLM_ERR_CUDA; the batch's
+ * states are then invalid for good (an instance's state cannot be set again).
+ * Without effect on operators that lack the symmetry of the reference
+ * tetrahedron, whose kernel has no such waits. */
+dglm_status dglm_batch_set_wait_limit(dglm_batch *b, long long cycles);
 long dglm_batch_kernel_launches(dglm_batch *b);
 size_t dglm_batch_device_bytes(dglm_batch *b);
 dglm_status dglm_batch_destroy(dglm_batch *b);

@@ -49,3 +49,22 @@ def test_symmetry_adapted_kernels(phys, N):
 def test_dense_pipelined_kernels(phys, N):
     v = [v for v, d in capi.variants(phys, N, "fp64") if d.startswith("pipe-dmma E=")][0]
     expire_and_recover(problem(phys, N), v)
+
+
+def test_batch_kernel():
+    """One instance per order: every order's tiles wait.  The states of a batch
+    whose wait ran out stay invalid; a new batch steps as before."""
+    probs = [P.advection_gaussian(n=4, N=N, width2=0.05) for N in (2, 3, 4, 5, 6)]
+    b = capi.BatchSolver(probs)
+    b.set_wait_limit(1)
+    b.step(1)
+    for _ in range(2):
+        with pytest.raises(capi.DglmError, match="bounded wait"):
+            b.sync()
+    b.close()
+    b = capi.BatchSolver(probs)
+    b.step(2)
+    b.sync()
+    for i, p in enumerate(probs):
+        assert rel(b.get_state(i), oracle.Oracle(p).run(2)[0]) < TOL
+    b.close()
