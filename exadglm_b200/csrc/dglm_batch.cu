@@ -31,6 +31,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -588,6 +589,7 @@ struct dglm_batch {
   bool sym = false;                 // all orders on the symmetry-adapted path
   BatchSymArgs sargs{};
   int *err = nullptr;
+  std::atomic<int> expired{-1};     // *err after the last dglm_batch_step (-1: not read yet)
   long long wait_cycles = kWaitCycles;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   long launches = 0;
@@ -1050,6 +1052,7 @@ dglm_status dglm_batch_step(dglm_batch *b, int nsteps) {
   if (nsteps < 0) return set_error(DGLM_ERR_INVALID, "dglm_batch_step: negative step count");
   DeviceGuard g(b->dev);
   b->launches = 0;
+  b->expired.store(-1);
   for (int i = 0; i < nsteps; i++) {
     const int c = b->cur;
     if (!b->graph[c]) {
@@ -1080,17 +1083,27 @@ dglm_status dglm_batch_step(dglm_batch *b, int nsteps) {
   return DGLM_OK;
 }
 
+// Waits for the batch's stream and reports an expired wait of the steps taken
+// so far.  The flag is read once per dglm_batch_step: a caller that takes every
+// instance's state out does not pay for it each time.
+static dglm_status batch_sync(dglm_batch *b, const char *what) {
+  int err = b->err ? b->expired.load() : 0;
+  const bool read = err < 0;
+  cudaError_t e = cudaSuccess;
+  if (read) e = cudaMemcpyAsync(&err, b->err, sizeof(int), cudaMemcpyDeviceToHost, b->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
+  if (e != cudaSuccess) return cuda_check(e, what);
+  if (read) b->expired.store(err);
+  if (err)
+    return set_error(DGLM_ERR_CUDA, std::string(what) + ": a bounded wait in the stage kernel "
+                                    "expired; results are invalid");
+  return DGLM_OK;
+}
+
 dglm_status dglm_batch_sync(dglm_batch *b) {
   if (!b) return set_error(DGLM_ERR_INVALID, "dglm_batch_sync: NULL batch");
   DeviceGuard g(b->dev);
-  cudaError_t e = cudaStreamSynchronize(b->stream);
-  int err = 0;
-  if (e == cudaSuccess && b->err)
-    e = cudaMemcpy(&err, b->err, sizeof(int), cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess && err)
-    return set_error(DGLM_ERR_CUDA, "dglm_batch_sync: a bounded wait in the stage kernel expired; "
-                                    "results are invalid");
-  return cuda_check(e, "dglm_batch_sync");
+  return batch_sync(b, "dglm_batch_sync");
 }
 
 int dglm_batch_count(dglm_batch *b) {
@@ -1109,8 +1122,8 @@ dglm_status dglm_batch_get_state(dglm_batch *b, int index, double *u, int on_dev
                                   sizeof(double) * (size_t)I.K * np_of(I.N),
                                   on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                                   b->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
-  return cuda_check(e, "dglm_batch_get_state");
+  if (e != cudaSuccess) return cuda_check(e, "dglm_batch_get_state");
+  return batch_sync(b, "dglm_batch_get_state");
 }
 
 dglm_status dglm_batch_get_time(dglm_batch *b, int index, double *t, double *dt, int *tstep) {
@@ -1120,9 +1133,9 @@ dglm_status dglm_batch_get_time(dglm_batch *b, int index, double *t, double *dt,
     return set_error(DGLM_ERR_INVALID, "dglm_batch_get_time: no such instance");
   DeviceGuard g(b->dev);
   BatchScalars s{};
-  cudaError_t e = cudaStreamSynchronize(b->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpy(&s, b->sc + index, sizeof(BatchScalars), cudaMemcpyDeviceToHost);
+  const dglm_status st = batch_sync(b, "dglm_batch_get_time");
+  if (st != DGLM_OK) return st;
+  cudaError_t e = cudaMemcpy(&s, b->sc + index, sizeof(BatchScalars), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return cuda_check(e, "dglm_batch_get_time");
   if (t) *t = s.t;
   if (dt) *dt = s.dt;

@@ -376,8 +376,9 @@ dglm_status dglm_batch_get_state(dglm_batch *b, int index, double *u, int on_dev
 dglm_status dglm_batch_get_time(dglm_batch *b, int index, double *t, double *dt, int *tstep);
 dglm_status dglm_batch_set_stream(dglm_batch *b, void *stream);
 /* Bound of the stage kernel's waits, as dglm_set_wait_limit for a handle.
- * After a wait ran out dglm_batch_sync returns DGLM_ERR_CUDA; the batch's
- * states are then invalid for good (an instance's state cannot be set again).
+ * After a wait ran out dglm_batch_sync, dglm_batch_get_state and
+ * dglm_batch_get_time return DGLM_ERR_CUDA; the batch's states are then
+ * invalid for good (an instance's state cannot be set again).
  * Without effect on operators that lack the symmetry of the reference
  * tetrahedron, whose kernel has no such waits. */
 dglm_status dglm_batch_set_wait_limit(dglm_batch *b, long long cycles);

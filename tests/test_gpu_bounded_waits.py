@@ -68,3 +68,17 @@ def test_batch_kernel():
     for i, p in enumerate(probs):
         assert rel(b.get_state(i), oracle.Oracle(p).run(2)[0]) < TOL
     b.close()
+
+
+def test_batch_states_and_times_are_refused_after_expiry():
+    """Without a sync in between, too: a caller may step and take the state."""
+    probs = [P.advection_gaussian(n=3, N=N, width2=0.05) for N in (3, 5)]
+    for take in (lambda b: b.get_state(1), lambda b: b.time(0)):
+        b = capi.BatchSolver(probs)
+        b.step(1)
+        take(b)   # read once: the next step's expiry is seen all the same
+        b.set_wait_limit(1)
+        b.step(1)
+        with pytest.raises(capi.DglmError, match="bounded wait"):
+            take(b)
+        b.close()
