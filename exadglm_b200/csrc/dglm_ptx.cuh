@@ -12,7 +12,11 @@ namespace dglm {
 // launch_pdl, so that one's start (barriers, the operator's copy to shared
 // memory) overlaps the end of the one before: each lets its successor start as
 // soon as all its blocks run, and reads nothing that an earlier kernel writes,
-// nor writes anything, before pdl_wait.
+// nor writes anything, before pdl_wait.  After it, too, what an earlier kernel
+// writes (states, register, penalties, wave speeds, scalars) is read by plain
+// loads only: __ldg, and const __restrict__ parameters, are for memory that
+// does not change while the kernel lives, which here begins under its
+// predecessor, and the compiler may move such loads across the wait.
 __device__ __forceinline__ void pdl_launch() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

@@ -774,12 +774,12 @@ __global__ void step_end_kernel(DevScalars *sc) {
 }
 
 // update_tau (euler_dglm.cpp:72-84)
-__global__ void tau_kernel(int K, double tau_scale, const int *__restrict__ vmapF,
-                           const double *__restrict__ maxv, double *__restrict__ tau) {
+__global__ void tau_kernel(int K, double tau_scale, const int *vmapF, const double *maxv,
+                           double *tau) {
   pdl_launch();
   pdl_wait();
   const long f = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (f < 4L * K) tau[f] = 0.25 * (maxv[f] + maxv[vmapF[f]]) * tau_scale;
+  if (f < 4L * K) tau[f] = 0.25 * (maxv[f] + maxv[__ldg(vmapF + f)]) * tau_scale;
 }
 
 // ---------------------------------------------------------------------------

@@ -117,11 +117,12 @@ __device__ __forceinline__ bool sym_adv_tile(const SymAdvOp &op, double *u, cons
 #pragma unroll
   for (int m = 0; m < MTT; m++) acc[m][0] = acc[m][1] = 0.0;
   double up[FH][4];
+  // (the state is written by the launch before: plain loads, see launch_pdl)
   auto gather = [&](int f, double (&x)[4]) {
-    x[0] = __ldg(ubase + nb[f].x);
-    x[1] = __ldg(ubase + nb[f].y);
-    x[2] = __ldg(ubase + nb[f].z);
-    x[3] = __ldg(ubase + nb[f].w);
+    x[0] = ubase[nb[f].x];
+    x[1] = ubase[nb[f].y];
+    x[2] = ubase[nb[f].z];
+    x[3] = ubase[nb[f].w];
   };
 #pragma unroll
   for (int f = 0; f < FH; f++) gather(f, up[f]);
@@ -250,7 +251,7 @@ __global__ void __launch_bounds__(32 * NW, 1)
 #pragma unroll
     for (int v = 0; v < 4; v++)
       s[v] = 0.5 * __ldg(a.fscale + (t * E + el) * 4 + fo[v]) *
-             __ldg(a.tau + (t * E + el) * 4 + fo[v]);
+             a.tau[(t * E + el) * 4 + fo[v]];
     ok = sym_adv_tile<C>(
         op, u, FlowRecord{F + lane, F + C::F_V + lane},
         reinterpret_cast<const int4 *>(F + C::F_V + C::F_W) + lane, a.u_in, s,
