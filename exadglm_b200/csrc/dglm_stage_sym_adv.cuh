@@ -110,7 +110,10 @@ __device__ __forceinline__ bool sym_adv_tile(const SymAdvOp &op, double *u, cons
       dmma(acc[mt0(3) + m], A[(mt0(3) + m) * 32], h3);
     }
   };
-  // neighbours, then the first traces: on their way under the volume k-steps
+  // neighbours, then the first traces: on their way under the volume k-steps.
+  // (The traces are asked for after two k-steps, which cover the latency of
+  // their addresses; before the first the warp waits for those: N=5, K=93,750
+  // 981 us per two steps against 924, N=6, K=63,888 1,222 against 1,152.)
   int4 nb[KSF];
 #pragma unroll
   for (int f = 0; f < KSF; f++) nb[f] = __ldg(P + f * 32);
@@ -124,17 +127,22 @@ __device__ __forceinline__ bool sym_adv_tile(const SymAdvOp &op, double *u, cons
     x[2] = ubase[nb[f].z];
     x[3] = ubase[nb[f].w];
   };
-#pragma unroll
-  for (int f = 0; f < FH; f++) gather(f, up[f]);
   if (!wait()) return false;
-#pragma unroll 4
-  for (int ks = 0; ks < KSV; ks++) {
+  auto volume = [&](int ks) {
     const int n = op.tvol[ks * 4 + l];
     const double u1 = uE[n & 0x3ff], u2 = uE[(n >> 10) & 0x3ff], u3 = uE[n >> 20];
     const double v1 = fl.vol(ks, 0), v2 = fl.vol(ks, 1), v3 = fl.vol(ks, 2);
     const double p3 = u3 * v3, sum = fma(u2, v2, p3), d = fma(u2, v2, -p3);
     mma(ks, fma(u1, v1, sum), fma(u1, v1, -sum), fma(-u1, v1, d), -fma(u1, v1, d));
-  }
+  };
+  constexpr int K0 = 2;
+  static_assert(K0 <= KSV, "k-steps before the gathers");
+#pragma unroll
+  for (int ks = 0; ks < K0; ks++) volume(ks);
+#pragma unroll
+  for (int f = 0; f < FH; f++) gather(f, up[f]);
+#pragma unroll 4
+  for (int ks = K0; ks < KSV; ks++) volume(ks);
   ahead();
   auto face = [&](int f, const double (&x)[4]) {
     // (padding positions repeat the last point: finite values, zero columns)
