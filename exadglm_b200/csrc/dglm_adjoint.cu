@@ -954,6 +954,7 @@ using namespace dglm;
 // ---------------------------------------------------------------------------
 
 struct AdjointTape {
+  dglm_handle *owner = nullptr;
   AdjVariant var{};
   int var_index = 0;
   long state = 0;            // doubles per stored state (nvar * vs)
@@ -1004,7 +1005,7 @@ dglm_status talloc(AdjointTape *t, std::vector<void *> &list, T **p, size_t coun
   const bool sized = &list == &t->sized;
   void *q = nullptr;
   const size_t n = std::max<size_t>(count * sizeof(T), 16);
-  cudaError_t e = cudaMalloc(&q, n);
+  cudaError_t e = handle_malloc(t->owner, &q, n);
   if (e != cudaSuccess) {
     *p = nullptr;
     return set_error(DGLM_ERR_NOMEM, std::string("adjoint: cudaMalloc of ") +
@@ -1027,6 +1028,7 @@ dglm_status tape_setup(dglm_handle *h) {
   if (h->tape && h->tape->AV) return DGLM_OK;
   free_tape(h);
   AdjointTape *t = new AdjointTape();
+  t->owner = h;
   h->tape = t;
   const std::vector<AdjVariant> &vl = adjoint_variants(h->d.physics, h->d.N);
   if (vl.empty()) {

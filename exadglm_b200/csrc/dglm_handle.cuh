@@ -18,7 +18,7 @@ struct dglm_handle {
   int run_variant = 0;            // launched: the selected one, or its fallback when the
                                   // uploaded operators lack the symmetry it needs
   dglm::StageVariantInfo vinfo{}; // of run_variant
-  bool op_symmetric = true;       // whether the uploaded operators have that symmetry
+  bool op_symmetric = false;      // whether the uploaded operators have that symmetry
   std::vector<double> Ahost;      // stacked [WDr WDs WDt -LIFT], Np x (3Np+NFF) row-major
   std::vector<double> sym_image;  // operator image of the symmetry-adapted kernel
   long vs = 0;                    // doubles between variables of a field
@@ -30,10 +30,13 @@ struct dglm_handle {
   double *AT = nullptr, *geo = nullptr, *fscale = nullptr, *nrm = nullptr;
   double *tau = nullptr, *maxv = nullptr, *vel = nullptr;
   int *vmapP = nullptr, *vmapF = nullptr, *Fmask = nullptr;
-  // per-element record [Kp][kRecord] (Euler handles but BF16x6): the 9 metrics,
-  // nx, ny, nz and Fscale of the 4 faces, one pad double; one bulk copy per
-  // tile in the tensor-memory and symmetry-adapted kernels
+  // record of the tensor-memory and symmetry-adapted kernels: [Kp][kRecord] per
+  // element (Euler: the 9 metrics, nx, ny, nz and Fscale of the 4 faces, one
+  // pad double; one bulk copy per tile) or the flow records (advection).  TF32x3
+  // and BF16x3 Euler handles always have it; FP64 handles have it while a
+  // symmetry-adapted variant runs and there is memory for it
   double *erec = nullptr;
+  size_t erec_bytes = 0;   // of an FP64 handle's
   // compact face maps (dglm_set_compact_face_maps), built from vmapP on first
   // use: per face the neighbour element and a code of its node list
   int *etoe = nullptr, *ftab = nullptr;
@@ -91,11 +94,25 @@ struct DeviceGuard {
   }
 };
 
+// Gives back the record of an FP64 handle's symmetry-adapted kernel, which then
+// runs on its fallback; false when there is none to give back.
+bool drop_record(dglm_handle *h);
+
+// cudaMalloc; where memory is short, with that record given back.
+inline cudaError_t handle_malloc(dglm_handle *h, void **q, size_t n) {
+  cudaError_t e = cudaMalloc(q, n);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    if (drop_record(h)) e = cudaMalloc(q, n);
+  }
+  return e;
+}
+
 template <typename T>
 inline dglm_status dalloc(dglm_handle *h, T **p, size_t count) {
   void *q = nullptr;
   const size_t n = count * sizeof(T);
-  cudaError_t e = cudaMalloc(&q, n ? n : 16);
+  cudaError_t e = handle_malloc(h, &q, n ? n : 16);
   if (e != cudaSuccess) {
     *p = nullptr;
     return set_error(DGLM_ERR_NOMEM, std::string("cudaMalloc failed: ") + cudaGetErrorString(e));

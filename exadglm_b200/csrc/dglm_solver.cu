@@ -396,12 +396,63 @@ dglm_status upload_operator_layout(dglm_handle *h) {
 
 // The variant to launch for the selected one: a symmetry-adapted variant needs
 // operators with the symmetry of the reference tetrahedron (every symmetric
-// node set's have it); others run on its fallback.
+// node set's have it) and its record; others run on its fallback.
 void choose_run_variant(dglm_handle *h) {
   StageVariantInfo v{};
   stage_variant_info(h->d.physics, h->d.N, h->variant, &v);
-  h->run_variant = v.mode == MODE_SYM && !h->op_symmetric ? v.fallback : h->variant;
+  const bool runs = v.mode != MODE_SYM || (h->op_symmetric && h->erec);
+  h->run_variant = runs ? h->variant : v.fallback;
   stage_variant_info(h->d.physics, h->d.N, h->run_variant, &h->vinfo);
+}
+
+void free_record(dglm_handle *h) {
+  cudaFree(h->erec);
+  h->bytes -= h->erec_bytes;
+  h->erec = nullptr;
+  h->erec_bytes = 0;
+}
+
+// Allocates the record where the selected variant takes one and the operators
+// allow it (an FP64 handle without memory for it runs on the fallback, as
+// before there was such a variant), or frees it; then chooses the variant to
+// launch.  True when the record is new and to be filled (fill_record).
+bool allocate_record(dglm_handle *h) {
+  bool fresh = false;
+  StageVariantInfo v{};
+  stage_variant_info(h->d.physics, h->d.N, h->variant, &v);
+  if (h->d.precision == DGLM_PREC_FP64) {
+    const bool want = v.mode == MODE_SYM && h->op_symmetric;
+    if (!want && h->erec) free_record(h);
+    if (want && !h->erec) {
+      const size_t n = sizeof(double) * (h->d.physics == DGLM_EULER
+                                             ? (size_t)kRecord * h->Kp
+                                             : sym_flow_doubles(h->d.N, h->d.K));
+      if (cudaMalloc((void **)&h->erec, n) == cudaSuccess) {
+        h->erec_bytes = n;
+        h->bytes += n;
+        fresh = true;
+      } else {
+        cudaGetLastError();
+        h->erec = nullptr;
+      }
+    }
+  }
+  choose_run_variant(h);
+  return fresh;
+}
+
+// Fills the record from the uploaded mesh (legacy stream; AT holds the operator
+// layout of the variant to launch).
+cudaError_t fill_record(dglm_handle *h) {
+  if (!h->erec) return cudaSuccess;
+  cudaError_t e =
+      h->d.physics == DGLM_EULER
+          ? launch_element_records(h->geo, h->nrm, h->fscale, h->Kp,
+                                   h->d.precision == DGLM_PREC_FP64, h->erec)
+          : launch_sym_flow(h->d.N, h->AT, h->geo, h->nrm, h->fscale, h->vel, h->vmapP, h->vs,
+                            h->Kp, h->d.K, h->erec);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+  return e;
 }
 
 // Brings the RK register into the run variant's order after a change of
@@ -478,6 +529,18 @@ dglm_status issue_step(dglm_handle *h, int cur, cudaStream_t s) {
 }
 
 }  // namespace
+
+bool dglm::drop_record(dglm_handle *h) {
+  if (h->d.precision != DGLM_PREC_FP64 || !h->erec) return false;
+  cudaStreamSynchronize(h->stream);
+  drop_graphs(h);   // the captured steps carry the pointer in their arguments
+  const int from_mode = h->vinfo.mode;
+  free_record(h);
+  choose_run_variant(h);
+  if (!h->mesh_ready || from_mode == h->vinfo.mode) return true;
+  dglm_status st = h->state_ready ? convert_register(h, from_mode) : DGLM_OK;
+  return st == DGLM_OK && upload_operator_layout(h) == DGLM_OK;
+}
 
 // Scratch of the one-off right-hand-side evaluations (dglm_rhs,
 // dglm_adjoint_rhs), allocated on first use.
@@ -566,10 +629,10 @@ dglm_status dglm_create(const dglm_desc *desc, dglm_handle **out) {
     if (st == DGLM_OK) st = s;
   };
   chk(dalloc(h, &h->AT, max_op_doubles(d.physics, d.N, h->Np, h->NFF)));
-  // the per-element record (Euler) follows the metrics in one allocation
-  const bool record = d.physics == DGLM_EULER && d.precision != DGLM_PREC_BF16X6;
-  chk(dalloc(h, &h->geo, (size_t)(9 + (record ? kRecord : 0)) * K));
-  if (record && h->geo) h->erec = h->geo + 9 * K;
+  chk(dalloc(h, &h->geo, (size_t)9 * K));
+  if (d.physics == DGLM_EULER &&
+      (d.precision == DGLM_PREC_TF32X3 || d.precision == DGLM_PREC_BF16X3))
+    chk(dalloc(h, &h->erec, (size_t)kRecord * K));
   chk(dalloc(h, &h->fscale, (size_t)4 * K));
   chk(dalloc(h, &h->nrm, (size_t)12 * K));
   chk(dalloc(h, &h->tau, (size_t)4 * K));
@@ -621,6 +684,7 @@ dglm_status dglm_destroy(dglm_handle *h) {
   for (cudaEvent_t ev : h->ens_ev)
     if (ev) cudaEventDestroy(ev);
   for (void *p : h->allocs) cudaFree(p);
+  if (h->d.precision == DGLM_PREC_FP64) cudaFree(h->erec);
   if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
   delete h;
   return DGLM_OK;
@@ -705,16 +769,15 @@ dglm_status dglm_upload_mesh(dglm_handle *h, const dglm_mesh_arrays *m) {
   const auto H2D = cudaMemcpyHostToDevice;
   h->op_symmetric = h->d.precision == DGLM_PREC_FP64 &&
                     sym_operator_image(h->d.N, h->Ahost.data(), m->Fmask, h->sym_image);
-  choose_run_variant(h);
+  // (until all of it is there, the handle has no mesh)
+  h->mesh_ready = h->state_ready = false;
+  allocate_record(h);
   drop_graphs(h);
   dglm_status os = upload_operator_layout(h);
   if (os != DGLM_OK) return os;
   cudaError_t e = cudaMemcpy(h->geo, geo.data(), sizeof(double) * geo.size(), H2D);
   if (e == cudaSuccess) e = cudaMemcpy(h->nrm, nrm.data(), sizeof(double) * nrm.size(), H2D);
   if (e == cudaSuccess) e = cudaMemcpy(h->fscale, m->Fscale, sizeof(double) * 4 * K, H2D);
-  if (e == cudaSuccess && h->erec)
-    e = launch_element_records(h->geo, h->nrm, h->fscale, Kp,
-                               h->d.precision == DGLM_PREC_FP64, h->erec);
   if (e == cudaSuccess) e = cudaMemcpy(h->vmapP, m->vmapP, sizeof(int) * K * NFF, H2D);
   if (e == cudaSuccess) e = cudaMemcpy(h->vmapF, m->vmapF, sizeof(int) * 4 * K, H2D);
   if (e == cudaSuccess) e = cudaMemcpy(h->Fmask, m->Fmask, sizeof(int) * NFF, H2D);
@@ -723,26 +786,7 @@ dglm_status dglm_upload_mesh(dglm_handle *h, const dglm_mesh_arrays *m) {
     for (int q = 0; q < 3 && e == cudaSuccess; q++)
       e = cudaMemcpy(h->vel + (size_t)q * h->vs, v3[q], sizeof(double) * K * Np, H2D);
   }
-  if (e == cudaSuccess && h->d.physics == DGLM_ADVECTION && h->op_symmetric) {
-    // flow records of the symmetry-adapted advection kernel, whatever variant
-    // is selected
-    if (!h->erec) {
-      dglm_status st = dalloc(h, &h->erec, sym_flow_doubles(h->d.N, h->d.K));
-      if (st != DGLM_OK) return st;
-    }
-    // (AT holds the operator image unless another variant is selected)
-    const bool other = h->vinfo.mode != MODE_SYM;
-    if (other)
-      e = cudaMemcpy(h->AT, h->sym_image.data(), sizeof(double) * h->sym_image.size(), H2D);
-    if (e == cudaSuccess)
-      e = launch_sym_flow(h->d.N, h->AT, h->geo, h->nrm, h->fscale, h->vel, h->vmapP, h->vs,
-                          h->Kp, h->d.K, h->erec);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
-    if (e == cudaSuccess && other) {
-      os = upload_operator_layout(h);
-      if (os != DGLM_OK) return os;
-    }
-  }
+  if (e == cudaSuccess) e = fill_record(h);
   if (e != cudaSuccess) return cuda_check(e, "dglm_upload_mesh");
   h->mesh_ready = true;
   h->state_ready = false;
@@ -1182,10 +1226,16 @@ dglm_status dglm_set_variant(dglm_handle *h, int variant) {
   drop_graphs(h);
   const int from_mode = h->vinfo.mode;
   h->variant = variant;
-  choose_run_variant(h);
-  if (!h->mesh_ready) return DGLM_OK;
+  if (!h->mesh_ready) {
+    choose_run_variant(h);
+    return DGLM_OK;
+  }
+  const bool fresh = allocate_record(h);
   dglm_status st = h->state_ready ? convert_register(h, from_mode) : DGLM_OK;
-  return st == DGLM_OK ? upload_operator_layout(h) : st;
+  if (st == DGLM_OK) st = upload_operator_layout(h);
+  if (st == DGLM_OK && fresh)
+    st = cuda_check(fill_record(h), "dglm_set_variant");
+  return st;
 }
 
 int dglm_get_variant(dglm_handle *h) { return h ? h->variant : -1; }

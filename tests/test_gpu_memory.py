@@ -1,0 +1,101 @@
+"""Device memory of FP64 handles: the record of the symmetry-adapted kernels is
+held only by handles that run them, and a handle gives it up (running on the
+dense fallback from then on) rather than fail where memory is short.
+
+The memory of the GPU is taken up by one tensor that leaves what the handle
+needs without the record and SLACK more (allocation granules and the kernels'
+code); the record of the mesh used is 234 MB."""
+import contextlib
+
+import numpy as np
+import pytest
+
+from exadglm_b200 import capi
+from exadglm_b200 import problem as P
+from exadglm_b200.mesh import Mesh3D, UniformBox
+
+pytestmark = pytest.mark.gpu
+
+SLACK = 96 << 20
+
+
+def sym_variant(phys, N):
+    return [v for v, d in capi.variants(phys, N, "fp64") if d.startswith("pipe-dmma-sym")][0]
+
+
+def solver(prob, variant):
+    return capi.Solver(prob, variant=variant)
+
+
+@contextlib.contextmanager
+def memory_left(leave):
+    """All device memory but `leave` bytes is taken."""
+    torch = pytest.importorskip("torch")
+    torch.cuda.empty_cache()
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - leave, dtype=torch.uint8, device="cuda")
+    yield
+    del hold
+    torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("phys,N", [("euler", 1), ("euler", 2), ("euler", 4), ("euler", 7),
+                                    ("advection", 2), ("advection", 5)])
+def test_only_handles_that_run_the_symmetry_adapted_kernels_hold_a_record(phys, N):
+    n = 3
+    prob = P.euler_sine(n=n, N=N) if phys == "euler" else P.advection_gaussian(n=n, N=N)
+    Np, Nfp, nvar, Kp = prob.Np, (N + 1) * (N + 2) // 2, prob.nvar, -(-prob.K // 64) * 64
+    fields = 3 * nvar + (3 if phys == "advection" else 0)
+    # fields, metrics, normals, Fscale, tau, maxv, and the maps
+    mesh = Kp * (8 * (fields * Np + 9 + 12 + 3 * 4) + 4 * (4 * Nfp + 4))
+    rest = 65536 * 8 + 4 * 4 * Nfp + 4096   # dt history, Fmask, scalars
+    dense = [v for v, d in capi.variants(phys, N, "fp64") if not d.startswith("pipe-dmma-sym")][0]
+    operators = 8 * 4 * (-(-Np // 8) * 8 + 8) * (3 * Np + 4 * Nfp + 32)   # any layout
+    s = solver(prob, -1)
+    has = N in ((3, 4, 5, 6) if phys == "euler" else (2, 3, 4, 5, 6))
+    s.set_variant(dense)
+    assert s.device_bytes() <= mesh + rest + operators
+    if has:
+        lean = s.device_bytes()
+        s.set_variant(sym_variant(phys, N))
+        assert s.device_bytes() > lean
+        s.set_variant(dense)
+        assert s.device_bytes() == lean
+    s.close()
+
+
+@pytest.fixture(scope="module")
+def big():
+    mesh = Mesh3D(5, UniformBox(26, 26, 26), high_order=False)
+    prob = P.advection_gaussian(N=5, width2=0.05, mesh=mesh)
+    dense = [v for v, d in capi.variants("advection", 5, "fp64")
+             if d.startswith("pipe-dmma E=16")][0]
+    s = solver(prob, dense)   # the fallback of the symmetry-adapted variant
+    lean = s.device_bytes()
+    s.step(2)
+    want = s.get_state()
+    s.close()
+    return prob, lean, want
+
+
+def test_no_memory_for_the_record(big):
+    prob, lean, want = big
+    with memory_left(lean + SLACK):
+        s = solver(prob, sym_variant("advection", 5))
+    assert s.device_bytes() == lean
+    s.step(2)
+    assert np.array_equal(s.get_state(), want)
+    s.close()
+
+
+def test_record_given_back_for_a_later_allocation(big):
+    """The ensemble's four state buffers (168 MB) do not fit beside it."""
+    prob, lean, want = big
+    s = solver(prob, sym_variant("advection", 5))
+    assert s.device_bytes() > lean + 2 * SLACK
+    s.step(1)
+    s.sync()
+    with memory_left(SLACK):
+        out = s.run_ensemble([prob.u0], 2)[0]
+    assert np.array_equal(out, want)
+    assert s.device_bytes() < lean + 4 * 8 * prob.K * prob.Np + (1 << 20)
+    s.close()
