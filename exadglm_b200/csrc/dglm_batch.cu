@@ -756,11 +756,10 @@ dglm_status finalize_sym(dglm_batch *b, const std::vector<BatchTile> &tiles,
     sum += kSymCost[tiles[i].N];
   }
   double *rec = nullptr;
-  int *dcut = nullptr, *lab = nullptr;
+  int *dcut = nullptr;
   const int **labels = nullptr;
   dglm_status st = balloc(b, &rec, (size_t)elems * kSymRec);
   if (st == DGLM_OK) st = balloc(b, &dcut, cut.size());
-  if (st == DGLM_OK) st = balloc(b, &lab, (size_t)4 * (kMaxOrder + 1));
   if (st == DGLM_OK) st = balloc(b, &labels, (size_t)kMaxOrder + 1);
   if (st == DGLM_OK) st = balloc(b, &b->err, 1);
   if (st != DGLM_OK) return st;
@@ -908,17 +907,9 @@ dglm_status dglm_batch_add(dglm_batch *b, int N, int K, const dglm_mesh_arrays *
   return DGLM_OK;
 }
 
-dglm_status dglm_batch_finalize(dglm_batch *b) {
-  if (!b) return set_error(DGLM_ERR_INVALID, "dglm_batch_finalize: NULL batch");
-  if (b->finalized) return set_error(DGLM_ERR_STATE, "dglm_batch_finalize: already finalized");
-  if (b->host.empty()) return set_error(DGLM_ERR_STATE, "dglm_batch_finalize: no instances");
-  DeviceGuard g(b->dev);
+// Uploads the instances for the path b->sym names and prepares their steps.
+static dglm_status finalize_path(dglm_batch *b, const std::vector<double> *image) {
   const int n = (int)b->host.size();
-  std::vector<double> image[kMaxOrder + 1];
-  b->sym = true;
-  for (int N = 2; N <= 6; N++)
-    if (!b->Ahost[N].empty())
-      b->sym = b->sym && sym_operator_image(N, b->Ahost[N].data(), b->Fm[N].data(), image[N]);
   long nodes = 0, elems = 0, fps = 0;
   b->hinst.resize(n);
   for (int i = 0; i < n; i++) {
@@ -1039,6 +1030,32 @@ dglm_status dglm_batch_finalize(dglm_batch *b) {
   e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
   if (e != cudaSuccess) return cuda_check(e, "dglm_batch_finalize");
+  return DGLM_OK;
+}
+
+dglm_status dglm_batch_finalize(dglm_batch *b) {
+  if (!b) return set_error(DGLM_ERR_INVALID, "dglm_batch_finalize: NULL batch");
+  if (b->finalized) return set_error(DGLM_ERR_STATE, "dglm_batch_finalize: already finalized");
+  if (b->host.empty()) return set_error(DGLM_ERR_STATE, "dglm_batch_finalize: no instances");
+  DeviceGuard g(b->dev);
+  std::vector<double> image[kMaxOrder + 1];
+  b->sym = true;
+  for (int N = 2; N <= 6; N++)
+    if (!b->Ahost[N].empty())
+      b->sym = b->sym && sym_operator_image(N, b->Ahost[N].data(), b->Fm[N].data(), image[N]);
+  dglm_status st = finalize_path(b, image);
+  if (st == DGLM_ERR_NOMEM && b->sym) {
+    // without memory for the symmetry-adapted path's lists and records: the
+    // dense kernel takes less
+    cudaGetLastError();
+    for (void *p : b->allocs) cudaFree(p);
+    b->allocs.clear();
+    b->bytes = 0;
+    b->err = nullptr;
+    b->sym = false;
+    st = finalize_path(b, image);
+  }
+  if (st != DGLM_OK) return st;
   b->host.clear();
   b->host.shrink_to_fit();
   b->cur = 0;

@@ -99,3 +99,28 @@ def test_record_given_back_for_a_later_allocation(big):
     assert np.array_equal(out, want)
     assert s.device_bytes() < lean + 4 * 8 * prob.K * prob.Np + (1 << 20)
     s.close()
+
+
+def test_batch_without_memory_for_the_symmetry_adapted_path():
+    """Its lists and records are 135 MB of the batch used.  (The two paths'
+    sums differ in their order: 1e-13 is the batch tests' bar.)"""
+    mesh = Mesh3D(6, UniformBox(25, 25, 25), high_order=False)
+    probs = [P.advection_gaussian(N=6, width2=w, mesh=mesh) for w in (0.05, 0.06, 0.07)]
+
+    def run():
+        b = capi.BatchSolver(probs)
+        b.step(2)
+        out = [b.get_state(i) for i in range(len(probs))]
+        nbytes = b.device_bytes()
+        b.close()
+        return out, nbytes
+
+    want, full = run()
+    K, Np, Nfp = probs[0].K, 84, 28
+    dense = 3 * K * (8 * (3 * Np + 25) + 16 * Nfp)   # states, register, geometry, vmapP
+    assert full > dense + SLACK
+    with memory_left(dense + SLACK):
+        got, lean = run()
+    assert lean < dense + (8 << 20)
+    for a, b in zip(got, want):
+        assert np.linalg.norm(a - b) <= 1e-13 * np.linalg.norm(b)
