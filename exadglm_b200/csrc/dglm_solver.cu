@@ -1015,9 +1015,16 @@ dglm_status dglm::run_steps(dglm_handle *h, int nsteps) {
 
 // Prescribed dt of the coming steps on the device (0: the CFL dt).  Written only
 // when it changes: the copy from pageable memory waits for the stream.
+// Refused while the stream is being captured: a step runs as a graph of its own,
+// and its capture would end the caller's.
 dglm_status dglm::set_dt_fixed(dglm_handle *h, double dt) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(h->stream, &cap);
+  if (e != cudaSuccess) return cuda_check(e, "dglm_step");
+  if (cap != cudaStreamCaptureStatusNone)
+    return set_error(DGLM_ERR_CUDA, "dglm_step: the handle's stream is being captured");
   if (h->dt_fixed == dt) return DGLM_OK;
-  cudaError_t e = cudaMemcpyAsync(&h->sc->dt_fixed, &dt, sizeof(double), cudaMemcpyHostToDevice,
+  e = cudaMemcpyAsync(&h->sc->dt_fixed, &dt, sizeof(double), cudaMemcpyHostToDevice,
                                   h->stream);
   // the pageable source must stay alive until the copy is staged
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
