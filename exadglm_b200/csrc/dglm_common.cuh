@@ -232,10 +232,10 @@ bool sym_operator_image(int N, const double *A, const int *Fmask, std::vector<do
 // vertex 0, grad r_a + sum_b grad r_b; normals times Fscale / 2, and Fscale / 2).
 cudaError_t launch_element_records(const double *geo, const double *nrm, const double *fscale,
                                    long Kp, bool sym, double *rec);
-// RK register of `tiles` tiles of 8 elements: nodal order (variable blocks of
-// vs doubles) to the kernel's fragment order, or back (out zeroed by the caller).
-void sym_reorder_register(int N, long tiles, int nvar, long vs, const double *in, double *out,
-                          bool to_sym);
+// RK register of K elements: nodal order (variable blocks of vs doubles) to the
+// kernel's fragment order, or back.
+cudaError_t launch_register_order(int N, int K, int nvar, long vs, const double *in, double *out,
+                                  bool to_sym, cudaStream_t s);
 
 // fused FP64 stage launcher (dglm_stage_fp64.cu)
 bool stage_fp64_supported(int physics, int N);

@@ -456,18 +456,19 @@ cudaError_t fill_record(dglm_handle *h) {
 }
 
 // Brings the RK register into the run variant's order after a change of
-// variant in the middle of a step (symmetry-adapted kernels keep it in
-// fragment order, the others in nodal order).  Host copies: a caller switches
-// variants between stages, if at all, once.
+// variant, which may come in the middle of a step (symmetry-adapted kernels
+// keep it in fragment order, the others in nodal order).  The state buffer that
+// is not current holds it meanwhile; the tails past the mesh stay zero.
 dglm_status convert_register(dglm_handle *h, int from_mode) {
-  if ((from_mode == MODE_SYM) == (h->vinfo.mode == MODE_SYM)) return DGLM_OK;
-  const size_t n = (size_t)h->nvar * h->vs;
-  std::vector<double> in(n), out(n, 0.0);
-  cudaError_t e = cudaMemcpy(in.data(), h->kreg, sizeof(double) * n, cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return cuda_check(e, "RK register");
-  sym_reorder_register(h->d.N, (h->d.K + 7) / 8, h->nvar, h->vs, in.data(), out.data(),
-                       h->vinfo.mode == MODE_SYM);
-  e = cudaMemcpy(h->kreg, out.data(), sizeof(double) * n, cudaMemcpyHostToDevice);
+  const bool to_sym = h->vinfo.mode == MODE_SYM;
+  if ((from_mode == MODE_SYM) == to_sym) return DGLM_OK;
+  const size_t bytes = sizeof(double) * h->nvar * h->vs;
+  double *tmp = h->u[h->cur ^ 1];
+  cudaError_t e = cudaMemcpyAsync(tmp, h->kreg, bytes, cudaMemcpyDeviceToDevice, h->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(h->kreg, 0, bytes, h->stream);
+  if (e == cudaSuccess)
+    e = launch_register_order(h->d.N, h->d.K, h->nvar, h->vs, tmp, h->kreg, to_sym, h->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(tmp, 0, bytes, h->stream);
   return cuda_check(e, "RK register");
 }
 

@@ -14,7 +14,7 @@ namespace dglm {
 namespace {
 
 // chi_c(a) of V4 with vertex i -> i^a: chi_1 = + on {0,1}, chi_2 on {0,2}, chi_3 on {0,3}
-int chi(int c, int a) { return c == 0 || a == 0 || a == c ? 1 : -1; }
+__host__ __device__ constexpr int chi(int c, int a) { return c == 0 || a == 0 || a == c ? 1 : -1; }
 
 // The node set of order N under V4 and the kernel's numbering of it.  Nodes
 // are in the datain order: the lattice (i_1, i_2, i_3) of barycentric counts,
@@ -243,44 +243,68 @@ bool build_image(const double *A, const int *Fmask, std::vector<double> &img) {
   return true;
 }
 
-// RK register between nodal (variable blocks of vs doubles) and fragment order.
+// nodes of chi_0's slots by label, for the register kernel
 template <int N>
-void reorder_register(long tiles, int nvar, long vs, const double *in, double *out, bool to_sym) {
+struct SlotNodes {
+  unsigned char n[SymSize<N>::R0][4];
+};
+
+// RK register between nodal (variable blocks of vs doubles) and fragment order:
+// a thread per (tile, variable, slot, MMA column), the slot's four characters.
+// Elements past K are zero in nodal order.
+template <int N>
+__global__ void register_order_kernel(SlotNodes<N> slots, long threads, int K, int nvar, long vs,
+                                      const double *__restrict__ in, double *__restrict__ out,
+                                      bool to_sym) {
   using Z = SymSize<N>;
-  const SymLayout<N> &L = sym_layout<N>();
   constexpr int Np = Z::Np, E = 8;
-  for (long t = 0; t < tiles; t++)
-    for (int v = 0; v < nvar; v++)
-      for (int e = 0; e < E; e++) {   // MMA columns
-        const long nod = v * vs + (t * E + Z::elem(e)) * Np, frag = (t * nvar + v) * Np * E + e;
-        for (int slot = 0; slot < Z::R0; slot++) {
-          const int *nd = L.slot_node[slot];
-          for (int c = 0; c < 4; c++) {
-            // the row of character c for this slot's orbit
-            int row = Z::krow(0, slot);
-            if (c > 0) {
-              if (slot < Z::N4) {
-                row = Z::krow(c, slot);
-              } else {
-                const int i = slot - Z::slot0(c, 0);
-                if (i < 0 || i >= Z::N2) continue;
-                row = Z::krow(c, Z::slotb(c, i));
-              }
-            }
-            const long f = frag + (long)row * E;
-            if (to_sym) {
-              out[f] = 0;
-              for (int a = 0; a < 4; a++) out[f] += 0.25 * chi(c, a) * in[nod + nd[a]];
-            } else {
-              for (int a = 0; a < 4; a++) {
-                bool first = true;   // a node that repeats in its orbit is added once
-                for (int q = 0; q < a; q++) first &= nd[q] != nd[a];
-                if (first) out[nod + nd[a]] += chi(c, a) * in[f];
-              }
-            }
-          }
-        }
-      }
+  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (i >= threads) return;
+  const int e = (int)(i % E), slot = (int)(i / E % Z::R0), v = (int)(i / (E * Z::R0) % nvar);
+  const long t = i / ((long)E * Z::R0 * nvar), k = t * E + Z::elem(e);
+  const long nod = v * vs + k * Np, frag = (t * nvar + v) * Np * E + e;
+  int nd[4], row[4];
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    nd[c] = slots.n[slot][c];
+    // the row of character c for this slot's orbit (-1: none)
+    const int q = slot - Z::slot0(c, 0);
+    row[c] = c == 0 || slot < Z::N4 ? Z::krow(c, slot)
+             : q >= 0 && q < Z::N2  ? Z::krow(c, Z::slotb(c, q))
+                                    : -1;
+  }
+  if (to_sym) {
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      double x = 0;
+#pragma unroll
+      for (int a = 0; a < 4; a++) x += chi(c, a) * in[nod + nd[a]];
+      if (row[c] >= 0) out[frag + (long)row[c] * E] = 0.25 * x;
+    }
+    return;
+  }
+  double y[4];
+#pragma unroll
+  for (int c = 0; c < 4; c++) y[c] = row[c] >= 0 ? in[frag + (long)row[c] * E] : 0.0;
+#pragma unroll
+  for (int a = 0; a < 4; a++) {   // (a node that repeats in its orbit gets equal values)
+    double x = 0;
+#pragma unroll
+    for (int c = 0; c < 4; c++) x += chi(c, a) * y[c];
+    out[nod + nd[a]] = k < K ? x : 0.0;
+  }
+}
+
+template <int N>
+cudaError_t register_order(int K, int nvar, long vs, const double *in, double *out, bool to_sym,
+                           cudaStream_t s) {
+  SlotNodes<N> slots;
+  for (int q = 0; q < SymSize<N>::R0; q++)
+    for (int a = 0; a < 4; a++) slots.n[q][a] = (unsigned char)sym_layout<N>().slot_node[q][a];
+  const long n = ((long)K + 7) / 8 * nvar * SymSize<N>::R0 * 8;
+  register_order_kernel<N><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(slots, n, K, nvar, vs, in,
+                                                                      out, to_sym);
+  return cudaGetLastError();
 }
 
 template <int N, int NS, int NG, int NB>
@@ -448,9 +472,11 @@ cudaError_t launch_sym_flow(int N, const double *image, const double *geo, const
   return e;
 }
 
-void sym_reorder_register(int N, long tiles, int nvar, long vs, const double *in, double *out,
-                          bool to_sym) {
-  SYM_ORDER(N, reorder_register<n>(tiles, nvar, vs, in, out, to_sym))
+cudaError_t launch_register_order(int N, int K, int nvar, long vs, const double *in, double *out,
+                                  bool to_sym, cudaStream_t s) {
+  cudaError_t e = cudaErrorInvalidValue;
+  SYM_ORDER(N, e = register_order<n>(K, nvar, vs, in, out, to_sym, s))
+  return e;
 }
 
 }  // namespace dglm
