@@ -366,11 +366,12 @@ struct SymWarp {
       s[v] = um + uv;
       d[v] = uv - um;
     }
+    // (velocities first, as in the dense kernels: the square of a momentum
+    // leaves the range of doubles long before the state does)
     const double ir = recip(s[0]);
     const double mn = nx * s[1] + ny * s[2] + nz * s[3];
-    const double vn = mn * ir;
-    const double p =
-        (gamma - 1) * (s[4] - 0.5 * (s[1] * s[1] + s[2] * s[2] + s[3] * s[3]) * ir);
+    const double vx = s[1] * ir, vy = s[2] * ir, vz = s[3] * ir, vn = mn * ir;
+    const double p = (gamma - 1) * (s[4] - 0.5 * (s[1] * vx + s[2] * vy + s[3] * vz));
 #pragma unroll
     for (int v = 0; v < NVW; v++) {
       const double fl = V0 + v == 0   ? mn
