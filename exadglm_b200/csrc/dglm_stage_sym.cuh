@@ -167,10 +167,13 @@ __device__ __forceinline__ void bulk_wait_read() {
 __device__ __forceinline__ void bulk_wait_all() {
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
-// 1/x by Newton's iteration from the hardware's approximation (two steps double
-// its ~20 bits twice; at most an ulp or so, branch-free).  x = 0, Inf and
-// denormals give NaN or 0: states that hold them are non-finite after the
-// update either way.
+// 1/x by Newton's iteration from the hardware's approximation, branch-free: two
+// steps take its 2^-23 below the rounding of the last, so the result is within
+// an ulp of the rounded quotient where x and 1/x are normal numbers.  Outside,
+// unlike the division: 0, subnormal numbers and infinities give NaN, and from
+// 2^1022 on the result is 0 (densities below 2.2e-308 or above 4.5e307).  With
+// 1.0 / x a step takes 5 % longer at N=3, 3.5 % at N=4, 7 % at N=5; with a range
+// check and a second pass with divisions for the tiles that fail it 1 to 3 %.
 __device__ __forceinline__ double recip(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));

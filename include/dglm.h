@@ -60,7 +60,9 @@ typedef enum { DGLM_ADVECTION = 0, DGLM_EULER = 1 } dglm_physics;
  * registers, the geometric factors and the face fluxes stay FP64 in every
  * mode. */
 typedef enum {
-    DGLM_PREC_FP64 = 0,        /* plain method: FP64 throughout */
+    DGLM_PREC_FP64 = 0,        /* plain method: FP64 throughout.  The Euler kernels of orders
+                                  3..6 ("pipe-dmma-sym") want densities between 2.3e-308 and
+                                  2.2e307; the other variants take any positive one */
     DGLM_PREC_TF32X3 = 1,      /* split TF32 (2 parts) on tcgen05, FP32 accumulate; the
                                   operator-in-tensor-memory kernel forms all 4 products */
     DGLM_PREC_BF16X3 = 2,      /* split BF16 (2 parts), 3 products (4 with the
