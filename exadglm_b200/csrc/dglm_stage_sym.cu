@@ -107,10 +107,11 @@ const SymLayout<N> &sym_layout() {
 
 // Largest deviation from the symmetry, of the largest entry, up to which the
 // operators' average over V4 stands for them.  The symmetry holds to rounding
-// for every node set that is symmetric itself (measured: 6e-15 at most for
-// orders 1..8); the bound is a few times that, of the size of the rounding
-// of the contraction itself.
-constexpr double kSymTol = 3e-14;
+// for every node set that is symmetric itself (orders 3..8 of this package: 1e-16
+// to 5.7e-15, with the linear algebra library's rounding; a set made elsewhere
+// may have some other); operators further off run on the dense kernels as they
+// are.
+constexpr double kSymTol = 1e-14;
 
 // face label v (0..3: opposite vertex v) -> face and its points' positions;
 // aligned: position pos[v][j] of face_of[v] is the image under v of point j

@@ -116,7 +116,11 @@ dglm_status dglm_create(const dglm_desc *desc, dglm_handle **out);
 dglm_status dglm_destroy(dglm_handle *h);
 dglm_status dglm_set_stream(dglm_handle *h, void *cuda_stream);
 /* Validates every index array on the host (0 <= vmapP < K*Np, 0 <= vmapF <
- * 4K, 0 <= Fmask < Np) and all real arrays for NaN/Inf, then uploads. */
+ * 4K, 0 <= Fmask < Np) and all real arrays for NaN/Inf, then uploads.  The
+ * FP64 kernels "pipe-dmma-sym" use the operators' average over the vertex
+ * permutations (01)(23), (02)(13), (03)(12) where they are that symmetric to
+ * 1e-14 of their largest entry; with others the handle runs on a dense
+ * variant. */
 dglm_status dglm_upload_mesh(dglm_handle *h, const dglm_mesh_arrays *mesh);
 /* u: nvar pointers to K*Np doubles (host or device per on_device).  Resets
  * t, tstep and the RK register k to zero and computes the face wave speeds
