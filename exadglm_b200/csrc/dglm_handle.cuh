@@ -123,6 +123,29 @@ inline dglm_status dalloc(dglm_handle *h, T **p, size_t count) {
   return DGLM_OK;
 }
 
+// Several arrays in one allocation (each 256-byte aligned): all of them are there
+// or none is, and an allocation takes some 0.2 ms whatever its size.
+struct Arrays {
+  struct Item {
+    void **p;
+    size_t at;
+  };
+  std::vector<Item> items;
+  size_t bytes = 0;
+  template <typename T>
+  void add(T **p, size_t count) {
+    items.push_back({reinterpret_cast<void **>(p), bytes});
+    bytes += (count * sizeof(T) + 255) / 256 * 256;
+  }
+  dglm_status allocate(dglm_handle *h) {
+    char *base = nullptr;
+    const dglm_status st = dalloc(h, &base, bytes);
+    if (st == DGLM_OK)
+      for (const Item &i : items) *i.p = base + i.at;
+    return st;
+  }
+};
+
 StageArgs stage_args(dglm_handle *h, const double *u_in, double *u_out, int s);
 void free_tape(dglm_handle *h);
 dglm_status run_steps(dglm_handle *h, int nsteps);

@@ -547,11 +547,13 @@ bool dglm::drop_record(dglm_handle *h) {
 // dglm_adjoint_rhs), allocated on first use.
 dglm_status dglm::ensure_rhs_scratch(dglm_handle *h) {
   if (h->rhs_in) return DGLM_OK;
-  dglm_status st = dalloc(h, &h->rhs_in, (size_t)h->nvar * h->vs);
-  if (st == DGLM_OK) st = dalloc(h, &h->rhs_out, (size_t)h->nvar * h->vs);
-  if (st == DGLM_OK) st = dalloc(h, &h->maxv_s, (size_t)4 * h->Kp);
-  if (st == DGLM_OK) st = dalloc(h, &h->tau_s, (size_t)4 * h->Kp);
-  if (st == DGLM_OK) st = dalloc(h, &h->sc_s, 1);
+  Arrays all;
+  all.add(&h->rhs_in, (size_t)h->nvar * h->vs);
+  all.add(&h->rhs_out, (size_t)h->nvar * h->vs);
+  all.add(&h->maxv_s, (size_t)4 * h->Kp);
+  all.add(&h->tau_s, (size_t)4 * h->Kp);
+  all.add(&h->sc_s, 1);
+  const dglm_status st = all.allocate(h);
   if (st != DGLM_OK) return st;
   // on the handle's stream, ordered before the copies that fill them
   cudaStream_t s = h->stream;

@@ -101,6 +101,34 @@ def test_record_given_back_for_a_later_allocation(big):
     s.close()
 
 
+def test_right_hand_side_without_memory_for_its_scratch(big):
+    """Half of the scratch would fit: each call is refused, and the first one
+    with the memory back works."""
+    torch = pytest.importorskip("torch")
+    prob, lean, _ = big
+    dense = [v for v, d in capi.variants("advection", 5, "fp64")
+             if d.startswith("pipe-dmma E=16")][0]
+    s = solver(prob, dense)
+    u = torch.from_numpy(prob.u0.copy()).cuda()
+    out, want = torch.zeros_like(u), torch.zeros_like(u)
+
+    def rhs(r):
+        s.rhs_device([u.data_ptr()], [r.data_ptr()])
+
+    with memory_left(64 << 20):
+        for _ in range(2):
+            with pytest.raises(capi.DglmError) as e:
+                rhs(out)
+            assert e.value.status == capi.ERR_NOMEM
+    assert s.device_bytes() == lean
+    rhs(out)
+    fresh = solver(prob, dense)
+    fresh.rhs_device([u.data_ptr()], [want.data_ptr()])
+    assert torch.equal(out, want) and float(out.abs().max()) > 0
+    s.close()
+    fresh.close()
+
+
 def test_batch_without_memory_for_the_symmetry_adapted_path():
     """Its lists and records are 135 MB of the batch used.  (The two paths'
     sums differ in their order: 1e-13 is the batch tests' bar.)"""
