@@ -626,30 +626,28 @@ dglm_status dglm_create(const dglm_desc *desc, dglm_handle **out) {
   h->Kp = ((long)d.K + 63) / 64 * 64;
   const long n = h->Kp * h->Np;
   h->vs = (n + 31) / 32 * 32;  // 256-byte aligned variable blocks
-  dglm_status st = DGLM_OK;
   const long K = h->Kp;
-  auto chk = [&](dglm_status s) {
-    if (st == DGLM_OK) st = s;
-  };
-  chk(dalloc(h, &h->AT, max_op_doubles(d.physics, d.N, h->Np, h->NFF)));
-  chk(dalloc(h, &h->geo, (size_t)9 * K));
+  Arrays all;
+  all.add(&h->AT, max_op_doubles(d.physics, d.N, h->Np, h->NFF));
+  all.add(&h->geo, (size_t)9 * K);
   if (d.physics == DGLM_EULER &&
       (d.precision == DGLM_PREC_TF32X3 || d.precision == DGLM_PREC_BF16X3))
-    chk(dalloc(h, &h->erec, (size_t)kRecord * K));
-  chk(dalloc(h, &h->fscale, (size_t)4 * K));
-  chk(dalloc(h, &h->nrm, (size_t)12 * K));
-  chk(dalloc(h, &h->tau, (size_t)4 * K));
-  chk(dalloc(h, &h->maxv, (size_t)4 * K));
+    all.add(&h->erec, (size_t)kRecord * K);
+  all.add(&h->fscale, (size_t)4 * K);
+  all.add(&h->nrm, (size_t)12 * K);
+  all.add(&h->tau, (size_t)4 * K);
+  all.add(&h->maxv, (size_t)4 * K);
   // padded to whole tiles: the tensor-core kernel bulk-copies vmapP per tile
-  chk(dalloc(h, &h->vmapP, (size_t)K * h->NFF));
-  chk(dalloc(h, &h->vmapF, (size_t)4 * K));
-  chk(dalloc(h, &h->Fmask, (size_t)h->NFF));
-  if (d.physics == DGLM_ADVECTION) chk(dalloc(h, &h->vel, (size_t)3 * h->vs));
-  chk(dalloc(h, &h->u[0], (size_t)h->nvar * h->vs));
-  chk(dalloc(h, &h->u[1], (size_t)h->nvar * h->vs));
-  chk(dalloc(h, &h->kreg, (size_t)h->nvar * h->vs));
-  chk(dalloc(h, &h->sc, 1));
-  chk(dalloc(h, &h->dt_hist, (size_t)kHistory));
+  all.add(&h->vmapP, (size_t)K * h->NFF);
+  all.add(&h->vmapF, (size_t)4 * K);
+  all.add(&h->Fmask, (size_t)h->NFF);
+  if (d.physics == DGLM_ADVECTION) all.add(&h->vel, (size_t)3 * h->vs);
+  all.add(&h->u[0], (size_t)h->nvar * h->vs);
+  all.add(&h->u[1], (size_t)h->nvar * h->vs);
+  all.add(&h->kreg, (size_t)h->nvar * h->vs);
+  all.add(&h->sc, 1);
+  all.add(&h->dt_hist, (size_t)kHistory);
+  dglm_status st = all.allocate(h);
   if (st == DGLM_OK) {
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess)
       st = set_error(DGLM_ERR_CUDA, "dglm_create: stream creation failed");
