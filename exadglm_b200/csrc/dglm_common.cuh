@@ -209,14 +209,16 @@ struct StageVariantInfo {
   int fallback;    // SYM: variant that runs when the operators lack the symmetry
 };
 
-// One entry of the variant tables: a tile shape and its launcher.
+// One entry of the variant tables: a tile shape and its launcher (and, where it
+// has one, its fallback's, by which the table finds the fallback's index).
 struct StageVariant {
   StageVariantInfo info;
   cudaError_t (*launch)(const StageArgs &, cudaStream_t);
+  cudaError_t (*fallback)(const StageArgs &, cudaStream_t) = nullptr;
 };
 
 // Symmetry-adapted stage (dglm_stage_sym.cu): Euler orders 3..6, advection 2..6.
-StageVariant sym_variant(int physics, int N, int fallback);
+StageVariant sym_variant(int physics, int N, const StageVariant &fallback);
 // Flow records of the advection kernel (dglm_stage_sym_adv.cuh): doubles for K
 // elements, and their making from the uploaded mesh (legacy stream).
 size_t sym_flow_doubles(int N, int K);

@@ -1028,17 +1028,35 @@ static const std::vector<Variant> &variants();
 #define DGLM_VARIANTS(P, NN, ...)                        \
   template <>                                            \
   const std::vector<Variant> &variants<P, NN>() {        \
-    static const std::vector<Variant> v = {__VA_ARGS__}; \
+    static const std::vector<Variant> v =                \
+        with_fallbacks({__VA_ARGS__});                   \
     return v;                                            \
   }
 
+// Fills in the fallbacks' indices: the entry that the variant names, else the
+// first plain FP64 one.
+static std::vector<Variant> with_fallbacks(std::vector<Variant> v) {
+  for (Variant &s : v) {
+    if (s.info.mode != MODE_SYM) continue;
+    s.info.fallback = -1;
+    for (int i = 0; i < (int)v.size(); i++) {
+      const StageVariantInfo &f = v[i].info;
+      if (f.mode == MODE_SYM || f.prec != DGLM_PREC_FP64) continue;
+      if (s.info.fallback < 0 || v[i].launch == s.fallback) s.info.fallback = i;
+    }
+  }
+  return v;
+}
+
 DGLM_VARIANTS(EUL, 1, V_SIMT(EUL, 1, 128, 4, 5), V_DMMA(EUL, 1, 64, 4, 1))
 DGLM_VARIANTS(EUL, 2, V_SIMT(EUL, 2, 64, 5, 5), V_DMMA(EUL, 2, 32, 4, 2))
-DGLM_VARIANTS(EUL, 3, sym_variant(EUL, 3, 4), V_DMMA(EUL, 3, 16, 2, 3), V_SIMT(EUL, 3, 32, 5, 5),
+DGLM_VARIANTS(EUL, 3, sym_variant(EUL, 3, V_PIPE(EUL, 3, 16, 1, 3, true)),
+              V_DMMA(EUL, 3, 16, 2, 3), V_SIMT(EUL, 3, 32, 5, 5),
               V_PIPE(EUL, 3, 8, 1, 3, true), V_PIPE(EUL, 3, 16, 1, 3, true),
               V_PIPEF(EUL, 3, 8, 1, true, 3, 2), V_PIPEF(EUL, 3, 16, 2, true, 3, 2),
               V_TC(EUL, 3, 8, 14, 3))
-DGLM_VARIANTS(EUL, 4, sym_variant(EUL, 4, 26), V_PIPE(EUL, 4, 8, 1, 2, true), V_DMMA(EUL, 4, 8, 1, 5),
+DGLM_VARIANTS(EUL, 4, sym_variant(EUL, 4, V_PIPEF(EUL, 4, 8, 1, true, 3, 2)),
+              V_PIPE(EUL, 4, 8, 1, 2, true), V_DMMA(EUL, 4, 8, 1, 5),
               V_SIMT(EUL, 4, 16, 5, 5), V_SIMT(EUL, 4, 16, 3, 5), V_DMMA(EUL, 4, 16, 1, 5),
               V_DMMA(EUL, 4, 16, 2, 5), V_PIPE(EUL, 4, 8, 1, 5, true),
               V_PIPE(EUL, 4, 8, 1, 5, false), V_PIPE(EUL, 4, 8, 1, 3, true),
@@ -1053,13 +1071,15 @@ DGLM_VARIANTS(EUL, 4, sym_variant(EUL, 4, 26), V_PIPE(EUL, 4, 8, 1, 2, true), V_
               V_PIPE2C(EUL, 4, 8, 5, 1, 2, 1), V_PIPE2C(EUL, 4, 8, 1, 5, 2, 2),
               V_TC(EUL, 4, 8, 14, 3), V_TCB(EUL, 4, 8, 14, 2, true),
               V_TC2(EUL, 4, 8, 13, 3), V_TCD(EUL, 4, 8, 14, 3))
-DGLM_VARIANTS(EUL, 5, sym_variant(EUL, 5, 10), V_PIPE(EUL, 5, 8, 1, 7, false), V_DMMA(EUL, 5, 8, 1, 7),
+DGLM_VARIANTS(EUL, 5, sym_variant(EUL, 5, V_PIPEFW(EUL, 5, 8, 5, 1, false, 2, 2)),
+              V_PIPE(EUL, 5, 8, 1, 7, false), V_DMMA(EUL, 5, 8, 1, 7),
               V_SIMT(EUL, 5, 8, 7, 5), V_M16(EUL, 5, 8, 1, 2, 2), V_M16(EUL, 5, 8, 1, 2, 1),
               V_M16(EUL, 5, 8, 1, 2, 3), V_PIPEF(EUL, 5, 8, 1, false, 3, 2),
               V_PM16G(EUL, 5, 8, 1, 2, 1, 2), V_PIPEFW(EUL, 5, 8, 5, 1, false, 1, 2),
               V_PIPEFW(EUL, 5, 8, 5, 1, false, 2, 2), V_PIPEFW(EUL, 5, 8, 5, 2, false, 3, 2),
               V_TCB(EUL, 5, 8, 14, 2, true), V_TCBD(EUL, 5, 8, 14, 2, true))
-DGLM_VARIANTS(EUL, 6, sym_variant(EUL, 6, 17), V_DMMA(EUL, 6, 8, 1, 6), V_SIMT(EUL, 6, 8, 7, 5),
+DGLM_VARIANTS(EUL, 6, sym_variant(EUL, 6, V_PIPEGW(EUL, 6, 8, 5, 2, 2, 1)),
+              V_DMMA(EUL, 6, 8, 1, 6), V_SIMT(EUL, 6, 8, 7, 5),
               V_PIPEG(EUL, 6, 8, 1, false, 2, 2), V_PIPEG(EUL, 6, 8, 1, false, 2, 1),
               V_PM16G(EUL, 6, 8, 1, 2, 1, 2), V_PM16G(EUL, 6, 8, 1, 2, 2, 2),
               V_PM16G(EUL, 6, 8, 1, 2, 3, 2),
@@ -1073,15 +1093,20 @@ DGLM_VARIANTS(EUL, 7, V_DMMA(EUL, 7, 8, 1, 5), V_SIMT(EUL, 7, 4, 8, 5))
 // N=8 Euler: the DMMA layout needs 8 elements per tile (40 columns), 242 KB
 DGLM_VARIANTS(EUL, 8, V_SIMT(EUL, 8, 4, 8, 5), V_SIMT(EUL, 8, 4, 6, 5))
 DGLM_VARIANTS(ADV, 1, V_SIMT(ADV, 1, 256, 4, 4), V_DMMA(ADV, 1, 64, 2, 1))
-DGLM_VARIANTS(ADV, 2, sym_variant(ADV, 2, 2), V_SIMT(ADV, 2, 128, 5, 4), V_DMMA(ADV, 2, 64, 2, 2))
-DGLM_VARIANTS(ADV, 3, sym_variant(ADV, 3, 7), V_DMMA(ADV, 3, 64, 2, 3), V_SIMT(ADV, 3, 64, 5, 4),
+DGLM_VARIANTS(ADV, 2, sym_variant(ADV, 2, V_DMMA(ADV, 2, 64, 2, 2)),
+              V_SIMT(ADV, 2, 128, 5, 4), V_DMMA(ADV, 2, 64, 2, 2))
+DGLM_VARIANTS(ADV, 3, sym_variant(ADV, 3, V_PIPEF(ADV, 3, 32, 1, true, 3, 2)),
+              V_DMMA(ADV, 3, 64, 2, 3), V_SIMT(ADV, 3, 64, 5, 4),
               V_PIPE(ADV, 3, 32, 1, 3, true), V_TF32(ADV, 3, 32), V_BF16(ADV, 3, 32),
               V_BF16X6(ADV, 3, 32, 8), V_PIPEF(ADV, 3, 32, 1, true, 3, 2))
-DGLM_VARIANTS(ADV, 4, sym_variant(ADV, 4, 3), V_SIMT(ADV, 4, 64, 5, 4), V_DMMA(ADV, 4, 64, 2, 5),
+DGLM_VARIANTS(ADV, 4, sym_variant(ADV, 4, V_PIPEF(ADV, 4, 32, 1, false, 3, 2)),
+              V_SIMT(ADV, 4, 64, 5, 4), V_DMMA(ADV, 4, 64, 2, 5),
               V_PIPEF(ADV, 4, 32, 1, false, 3, 2))
-DGLM_VARIANTS(ADV, 5, sym_variant(ADV, 5, 3), V_SIMT(ADV, 5, 32, 7, 4), V_DMMA(ADV, 5, 32, 1, 7),
+DGLM_VARIANTS(ADV, 5, sym_variant(ADV, 5, V_PIPEF(ADV, 5, 16, 1, false, 4, 2)),
+              V_SIMT(ADV, 5, 32, 7, 4), V_DMMA(ADV, 5, 32, 1, 7),
               V_PIPEF(ADV, 5, 16, 1, false, 4, 2))
-DGLM_VARIANTS(ADV, 6, sym_variant(ADV, 6, 4), V_SIMT(ADV, 6, 32, 7, 4), V_DMMA(ADV, 6, 32, 1, 6),
+DGLM_VARIANTS(ADV, 6, sym_variant(ADV, 6, V_PIPEF(ADV, 6, 8, 1, false, 12, 2)),
+              V_SIMT(ADV, 6, 32, 7, 4), V_DMMA(ADV, 6, 32, 1, 6),
               V_PIPEF(ADV, 6, 8, 1, false, 8, 2), V_PIPEF(ADV, 6, 8, 1, false, 12, 2),
               V_M16(ADV, 6, 32, 1, 2, 2), V_M16(ADV, 6, 32, 1, 2, 1),
               V_M16(ADV, 6, 32, 1, 2, 3), V_PM16G(ADV, 6, 16, 1, 2, 1, 2),

@@ -332,7 +332,7 @@ cudaError_t launch_sym(const StageArgs &a, cudaStream_t s) {
 }
 
 template <int N, int NS, int NG, int NB>
-StageVariant make_sym(int fallback) {
+StageVariant make_sym(const StageVariant &fallback) {
   using C = SymCfg<N, NS, NG, NB>;
   StageVariantInfo i{};
   i.mode = MODE_SYM;
@@ -344,8 +344,7 @@ StageVariant make_sym(int fallback) {
   i.R = C::WPG;
   i.ring = NB;
   i.persistent = 1;
-  i.fallback = fallback;
-  return StageVariant{i, &launch_sym<N, NS, NG, NB>};
+  return StageVariant{i, &launch_sym<N, NS, NG, NB>, fallback.launch};
 }
 
 template <int N, int NW>
@@ -364,7 +363,7 @@ cudaError_t launch_sym_adv(const StageArgs &a, cudaStream_t s) {
 }
 
 template <int N, int NW>
-StageVariant make_sym_adv(int fallback) {
+StageVariant make_sym_adv(const StageVariant &fallback) {
   using C = SymAdvCfg<N, NW>;
   StageVariantInfo i{};
   i.mode = MODE_SYM;
@@ -376,8 +375,7 @@ StageVariant make_sym_adv(int fallback) {
   i.R = 1;
   i.ring = 2;
   i.persistent = 1;
-  i.fallback = fallback;
-  return StageVariant{i, &launch_sym_adv<N, NW>};
+  return StageVariant{i, &launch_sym_adv<N, NW>, fallback.launch};
 }
 
 template <int N>
@@ -420,7 +418,7 @@ cudaError_t launch_element_records(const double *geo, const double *nrm, const d
   return cudaGetLastError();
 }
 
-StageVariant sym_variant(int physics, int N, int fallback) {
+StageVariant sym_variant(int physics, int N, const StageVariant &fallback) {
   // Warps per CTA: what the registers allow, less where the shared memory they
   // take is better left to L1 for the gathers (N=6, K=63,888: 8 warps 0.125 ms
   // per stage, 12 warps 0.154; N=3, K=162,000: 24 0.057, 16 0.059, 12 0.063;
