@@ -45,6 +45,7 @@
 
 #include "dglm_common.cuh"
 #include "dglm_handle.cuh"
+#include "dglm_ptx.cuh"
 
 namespace dglm {
 
@@ -379,13 +380,6 @@ __global__ void __launch_bounds__(ACfg<PHYS, N, E_>::T, MINB)
 // element-local phases (Jacobians, faces, update), which use all threads.
 // ---------------------------------------------------------------------------
 
-__device__ __forceinline__ void adj_dmma(double (&d)[2], double a, double b) {
-  asm volatile(
-      "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-      : "+d"(d[0]), "+d"(d[1])
-      : "d"(a), "d"(b));
-}
-
 // Face terms of the adjoint stage, one thread per face point p = e NFF + fj
 // (the face loop of the fused kernels, split out so that its gathers -- the
 // partner trace u[vmapP], phi at p and at the partner point mapP[p], and the
@@ -507,7 +501,7 @@ __device__ __forceinline__ void adj_contract_all_n(const double *A, int MTX, int
       const double av = an[ks % PF];
       if (ks + PF < C::KS) an[ks % PF] = __ldg(Ab + (long)(ks + PF) * MTX * 32);
 #pragma unroll
-      for (int j = 0; j < NT; j++) adj_dmma(acc[j], av, Bb[ks * 4 * C::BLD + j * 8]);
+      for (int j = 0; j < NT; j++) dmma_8x8x4(acc[j], av, Bb[ks * 4 * C::BLD + j * 8]);
     }
     const int row = mt * 8 + (lane >> 2);
     if (row < rows) {
@@ -679,7 +673,7 @@ __global__ void __launch_bounds__(DCfg<PHYS, N, E_, MG_, SPLIT>::T, MINB)
       const double bv = Bb[ks * 4 * BLD];
 #pragma unroll
       for (int i = 0; i < C::WMV; i++)
-        if (m0 + i < C::MTV) adj_dmma(acc[i], __ldg(Ab + ((long)ks * C::MTV + i) * 32), bv);
+        if (m0 + i < C::MTV) dmma_8x8x4(acc[i], __ldg(Ab + ((long)ks * C::MTV + i) * 32), bv);
     }
     // results -> sOut[row][v][e] (row = d*Np + j)
 #pragma unroll
@@ -775,7 +769,7 @@ __global__ void __launch_bounds__(DCfg<PHYS, N, E_, MG_, SPLIT>::T, MINB)
       const double bv = Bb[ks * 4 * BLD];
 #pragma unroll
       for (int i = 0; i < C::WML; i++)
-        if (m0 + i < C::MTL) adj_dmma(acc[i], __ldg(Ab + ((long)ks * C::MTL + i) * 32), bv);
+        if (m0 + i < C::MTL) dmma_8x8x4(acc[i], __ldg(Ab + ((long)ks * C::MTL + i) * 32), bv);
     }
 #pragma unroll
     for (int i = 0; i < C::WML; i++) {

@@ -120,13 +120,6 @@ __device__ __forceinline__ void b_cp_wait() {
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-__device__ __forceinline__ void b_dmma(double (&d)[2], double a, double b) {
-  asm volatile(
-      "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-      : "+d"(d[0]), "+d"(d[1])
-      : "d"(a), "d"(b));
-}
-
 template <int N>
 __device__ __forceinline__ void batch_tile(const BatchArgs &a, const BatchTile &t,
                                            double *smem) {
@@ -221,7 +214,7 @@ __device__ __forceinline__ void batch_tile(const BatchArgs &a, const BatchTile &
       const double *Bb = sB + (lane & 3) * BLD + nt * 8 + (lane >> 2);
 #pragma unroll 4
       for (int ks = 0; ks < C::KVP / 4; ks++)
-        b_dmma(acc[j], __ldg(Ab + (long)ks * C::MT * 32), Bb[ks * 4 * BLD]);
+        dmma_8x8x4(acc[j], __ldg(Ab + (long)ks * C::MT * 32), Bb[ks * 4 * BLD]);
     }
   }
   __syncthreads();
@@ -252,7 +245,7 @@ __device__ __forceinline__ void batch_tile(const BatchArgs &a, const BatchTile &
       const double *Bb = sB + (lane & 3) * BLD + nt * 8 + (lane >> 2);
 #pragma unroll 4
       for (int ks = 0; ks < C::KFP / 4; ks++)
-        b_dmma(acc[j], __ldg(Ab + (long)ks * C::MT * 32), Bb[ks * 4 * BLD]);
+        dmma_8x8x4(acc[j], __ldg(Ab + (long)ks * C::MT * 32), Bb[ks * 4 * BLD]);
     }
   }
   __syncthreads();

@@ -394,6 +394,13 @@ dglm_status upload_operator_layout(dglm_handle *h) {
                     "operator upload");
 }
 
+bool has_symmetric_variant(const dglm_handle *h) {
+  StageVariantInfo v{};
+  for (int i = 0; stage_variant_info(h->d.physics, h->d.N, i, &v); i++)
+    if (v.mode == MODE_SYM && v.prec == h->d.precision) return true;
+  return false;
+}
+
 // The variant to launch for the selected one: a symmetry-adapted variant needs
 // operators with the symmetry of the reference tetrahedron (every symmetric
 // node set's have it) and its record; others run on its fallback.
@@ -768,7 +775,7 @@ dglm_status dglm_upload_mesh(dglm_handle *h, const dglm_mesh_arrays *m) {
   cudaStreamSynchronize(h->stream);
   free_tape(h);   // the adjoint's operators and face pairing belong to the old mesh
   const auto H2D = cudaMemcpyHostToDevice;
-  h->op_symmetric = h->d.precision == DGLM_PREC_FP64 &&
+  h->op_symmetric = has_symmetric_variant(h) &&
                     sym_operator_image(h->d.N, h->Ahost.data(), m->Fmask, h->sym_image);
   // (until all of it is there, the handle has no mesh)
   h->mesh_ready = h->state_ready = false;
