@@ -335,9 +335,9 @@ using BSC = SymAdvCfg<N, sym_warps<N>()>;
 constexpr size_t kBatchSymSmem =
     cmax(cmax(cmax(BSC<2>::SMEM, BSC<3>::SMEM), cmax(BSC<4>::SMEM, BSC<5>::SMEM)),
          BSC<6>::SMEM) + 16 * kSymWarps;
-// Cost of a tile of order N (measured ns of a device's stage per tile), the
+// Cost of a tile of order N (a single mesh's stage over its tiles, in ns), the
 // weight by which the stretches are cut.
-constexpr double kSymCost[7] = {0, 0, 1.7, 2.9, 4.6, 8.3, 15.7};
+constexpr double kSymCost[7] = {0, 0, 1.6, 2.7, 4.2, 7.5, 13.9};
 
 // Tiles [lo, hi) of order N by this CTA.  it: buffer uses of the warp so far.
 template <int N>

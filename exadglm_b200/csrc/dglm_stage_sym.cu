@@ -419,13 +419,14 @@ cudaError_t launch_element_records(const double *geo, const double *nrm, const d
 }
 
 StageVariant sym_variant(int physics, int N, const StageVariant &fallback) {
-  // Warps per CTA: what the registers allow, less where the shared memory they
-  // take is better left to L1 for the gathers (N=6, K=63,888: 8 warps 0.125 ms
-  // per stage, 12 warps 0.154; N=3, K=162,000: 24 0.057, 16 0.059, 12 0.063;
-  // N=5, K=93,750: 16 0.092, 12 0.097, 20 0.111).  Against the dense kernels:
-  // N=2, K=384,000 0.307 -> 0.080, N=3 0.097 -> 0.057, N=4, K=105,456 0.117 ->
-  // 0.061, N=5 0.236 -> 0.092 (58 % of the HBM copy rate for its bytes), N=6
-  // 0.254 -> 0.125.
+  // Warps per CTA: what the registers allow (N=3 spills 4 bytes), less where the
+  // shared memory they take is better left to L1 for the gathers (ms per stage,
+  // counted with the gathers before the first k-step: N=6, K=63,888: 8 warps
+  // 0.125, 12 warps 0.154; N=3, K=162,000: 24 0.057, 16 0.059, 12 0.063; N=5,
+  // K=93,750: 16 0.092, 12 0.097, 20 0.111).  Against the dense kernels: N=2,
+  // K=384,000 0.313 -> 0.077, N=3 0.096 -> 0.054, N=4, K=105,456 0.118 -> 0.056,
+  // N=5 0.235 -> 0.088 (4.4 TB/s of HBM traffic, 67 % of the copy rate), N=6
+  // 0.254 -> 0.111.
   if (physics == DGLM_ADVECTION) switch (N) {
     case 2: return make_sym_adv<2, 16>(fallback);
     case 3: return make_sym_adv<3, 24>(fallback);

@@ -36,13 +36,14 @@
 //   k        the RK register is kept in fragment order (tile, variable,
 //            operator row, column): compute warps load and store it straight
 //            from registers, in full sectors.
-// Bound by (N=4, K=196,608): nothing alone.  The FP64 pipe (MMAs and fluxes)
-// needs 2.1k cycles per tile and HBM 2.2k; a tile takes 4.7k, where the warps
-// wait on shared memory (a third of it the update's and the traces' scattered
-// nodes), on the shared FP64 pipe (a warp's flux arithmetic gets one slot per
-// MMA of the other's) and on each other.  0.398 ms per stage against 0.782 of
-// the dense pipelined kernel; N=3 (K=105,456) 0.138 against 0.201, N=5
-// (K=82,944) 0.434 against 0.674, N=6 (K=82,944) 0.793 against 1.243.
+// Bound by (N=4, K=196,608): nothing alone.  The FP64 pipe needs 2.4k cycles per
+// tile (MMAs 1.4k, flux arithmetic 1.0k: counters of profiles/) and HBM 2.0k; a
+// tile takes 4.7k, where the warps wait on shared memory (a third of it the
+// update's and the traces' scattered nodes), on the shared FP64 pipe (a warp's
+// flux arithmetic gets one slot per MMA of the other's) and on each other.
+// 0.399 ms per stage against 0.780 of the dense pipelined kernel; N=3
+// (K=105,456) 0.136 against 0.201, N=5 (K=82,944) 0.420 against 0.674, N=6
+// (K=82,944, where a thread spills 100 bytes) 0.800 against 1.243.
 // Measured and not kept: each warp on its own tile with the traces gathered
 // into registers (0.698; the gathers stall the load path), one warp of the pair
 // on the volume k-steps and the other on faces and update (0.53), twelve
