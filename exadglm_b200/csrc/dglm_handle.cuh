@@ -123,10 +123,9 @@ inline dglm_status dalloc(dglm_handle *h, T **p, size_t count) {
   return DGLM_OK;
 }
 
-// Several arrays that are all there or not at all.  In one allocation (each
-// 256-byte aligned), which takes some 0.3 ms whatever its size; one by one where
-// all are below 1 MiB, because the driver cuts such pieces out of memory that it
-// holds (some 0.01 ms each).
+// Several arrays that are all there or not at all.  Those of 1 MiB and more share
+// one allocation (each 256-byte aligned), which takes some 0.3 ms whatever its
+// size; the driver cuts smaller ones out of memory that it holds (0.01 ms).
 struct Arrays {
   struct Item {
     void **p;
@@ -138,33 +137,32 @@ struct Arrays {
     items.push_back({reinterpret_cast<void **>(p), (count * sizeof(T) + 255) / 256 * 256});
   }
   dglm_status allocate(dglm_handle *h) {
-    size_t total = 0, largest = 0, done = 0;
+    constexpr size_t kLarge = 1u << 20;
+    const size_t before = h->allocs.size();
+    size_t shared = 0, taken = 0;
     for (const Item &i : items) {
-      total += i.bytes;
-      largest = i.bytes > largest ? i.bytes : largest;
+      *i.p = nullptr;
+      if (i.bytes >= kLarge) shared += i.bytes;
     }
     char *base = nullptr;
-    dglm_status st = DGLM_OK;
-    if (largest >= (1u << 20)) {
-      st = dalloc(h, &base, total);
-      for (const Item &i : items) {
+    dglm_status st = shared ? dalloc(h, &base, shared) : DGLM_OK;
+    if (st == DGLM_OK) taken = shared;
+    for (const Item &i : items) {
+      if (st != DGLM_OK) break;
+      if (i.bytes >= kLarge) {
         *i.p = base;
-        if (base) base += i.bytes;
+        base += i.bytes;
+        continue;
       }
-      return st;
+      char *own = nullptr;
+      st = dalloc(h, &own, i.bytes);
+      *i.p = own;
+      if (st == DGLM_OK) taken += i.bytes;
     }
-    for (; done < items.size() && st == DGLM_OK; done++) {
-      st = dalloc(h, &base, items[done].bytes);
-      *items[done].p = base;
-    }
-    for (; st != DGLM_OK && done-- > 0;) {
-      void *p = *items[done].p;
-      *items[done].p = nullptr;
-      if (!p) continue;   // the one that failed
-      cudaFree(p);
-      h->allocs.pop_back();
-      h->bytes -= items[done].bytes;
-    }
+    if (st == DGLM_OK) return st;
+    for (; h->allocs.size() > before; h->allocs.pop_back()) cudaFree(h->allocs.back());
+    h->bytes -= taken;
+    for (const Item &i : items) *i.p = nullptr;
     return st;
   }
 };
