@@ -129,6 +129,36 @@ def test_right_hand_side_without_memory_for_its_scratch(big):
     fresh.close()
 
 
+def test_record_given_back_between_two_stages():
+    """Euler N=4, K=196,608: the element record is 41 MB, and the right-hand side's
+    scratch (563 MB) is asked for after the first of five stages, with 24 MB less
+    than it needs.  The other stages run on the fallback, from the register as
+    the first left it: the state of five stages on one kernel, to rounding."""
+    torch = pytest.importorskip("torch")
+    prob = P.euler_sine(n=32, N=4)
+    variant = sym_variant("euler", 4)
+    scratch = 8 * (2 * 5 * 35 + 2 * 4) * prob.K
+    states = []
+    for squeeze in (False, True):
+        s = solver(prob, variant)
+        s.step(1)   # wave speeds and tau for the stages
+        dt = s.time()[1]
+        s.stage(0, dt)
+        if squeeze:
+            u = torch.from_numpy(prob.u0.copy()).cuda()
+            r = torch.empty_like(u)
+            before = s.device_bytes()
+            with memory_left(scratch - (24 << 20)):
+                s.rhs_device([x.data_ptr() for x in u], [x.data_ptr() for x in r])
+            assert s.device_bytes() - before < scratch - (32 << 20)   # the record is gone
+        for st in range(1, 5):
+            s.stage(st, dt)
+        states.append(s.get_state())
+        s.close()
+    a, b = states
+    assert np.linalg.norm(a - b) <= 1e-14 * np.linalg.norm(b)
+
+
 def test_batch_without_memory_for_the_symmetry_adapted_path():
     """Its lists and records are 135 MB of the batch used.  (The two paths'
     sums differ in their order: 1e-13 is the batch tests' bar.)"""
